@@ -359,6 +359,11 @@ void check_common(const DeviceOperator& op, const double* d_b, const SolveOption
         throw std::invalid_argument("failure_probability must lie strictly between zero and one");
 }
 
+int resident_sms(const SolveOptions& o) {
+    if (o.resident_sms >= 0) return o.resident_sms;
+    return o.use_graphs ? sm_count() : 0;
+}
+
 // Candidate bookkeeping: three device solution buffers so that the latest
 // and the best candidate survive without copies.
 struct Candidate {
@@ -483,7 +488,7 @@ SolveResult solve_amfls(const DeviceOperator& op, const double* d_b, const Solve
     const long long launches0 = launch_count();
     Statistics stats;
     Workspace ws(op, d_b, reg, o.maximum_basis_size, stream, o.time_operators,
-                 o.use_graphs && op.graph_safe(), o.reduced_basis);
+                 o.use_graphs && op.graph_safe(), o.reduced_basis, resident_sms(o));
     Evaluator ev(ws, op, d_b, reg, stats, stream);
     long long seen[4] = {0, 0, 0, 0};
     auto absorb = [&] {
@@ -821,7 +826,7 @@ SolveResult solve_fixed_rbgk(const DeviceOperator& op, const double* d_b, const 
     const long long launches0 = launch_count();
     Statistics stats;
     Workspace ws(op, d_b, reg, o.maximum_basis_size, stream, o.time_operators,
-                 o.use_graphs && op.graph_safe(), o.reduced_basis);
+                 o.use_graphs && op.graph_safe(), o.reduced_basis, resident_sms(o));
     Evaluator ev(ws, op, d_b, reg, stats, stream);
     long long seen[4] = {0, 0, 0, 0};
     auto absorb = [&] {

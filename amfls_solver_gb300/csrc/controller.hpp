@@ -26,6 +26,9 @@ struct SolveOptions {
     bool stop_early = true;   // fixed RBGK only
     bool time_operators = true;
     bool use_graphs = true;
+    // SMs the resident level kernel may take: -1 all of them when use_graphs
+    // (else none), 0 none; a batch gives each problem its share.
+    int resident_sms = -1;
     // At a work or basis limit return the latest checkpoint's candidate even
     // for lambda = 0 (the reference returns the one with the smallest
     // backward error there, amfls.cpp:156-163).  Not part of the reference's

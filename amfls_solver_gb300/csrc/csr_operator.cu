@@ -41,6 +41,8 @@
 #include "dd.cuh"
 #include "epilogue.cuh"
 #include "fp_bounds.cuh"
+#include "resident_levels.hpp"
+#include "sliced_rows.cuh"
 
 namespace amfls_gpu {
 
@@ -559,6 +561,19 @@ constexpr double kTuneMargin = 0.10;
 // runs).
 constexpr double kVectorMargin = 0.05;
 
+// Operators of at most this many nonzeros carry the sliced-row copy that the
+// resident level kernel multiplies by (two sides of 12 bytes a nonzero, up to
+// a quarter more for padding: 4 GB at the limit), where it takes at most half
+// of the free memory.  It pays at every size measured, up to the 40 million
+// nonzeros of the 2M x 500k matrix; beyond the limit the kernel chain runs.
+constexpr long long kResidentMaxNonzeros = 1LL << 27;
+
+bool sliced_rows_fit(long long nnz) {
+    size_t free_bytes = 0, total = 0;
+    AMFLS_CUDA(cudaMemGetInfo(&free_bytes, &total));
+    return nnz <= kResidentMaxNonzeros && 2 * 30 * (size_t)nnz <= free_bytes;
+}
+
 struct CsrOperator::Side {
     long long* off = nullptr;  // count+1
     int* off32 = nullptr;      // count+1, padded (bulk-copy source)
@@ -576,6 +591,7 @@ struct CsrOperator::Side {
     csr_vector::Table vtab{};
     bool vector = false;
     double vector_us = 0.0;
+    sliced::Store rows;  // products of the resident level kernel
 };
 
 namespace {
@@ -696,6 +712,7 @@ void CsrOperator::release() {
         s->off32 = nullptr;
         s->one.release();
         s->many.release();
+        s->rows.release();
         cudaFree(s->vrows);
         s->vrows = nullptr;
     }
@@ -825,6 +842,10 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
     AMFLS_CUDA(cudaStreamSynchronize(stream));
     if (err & 4) fail("CSR column index is out of range");
     if (err & 8) fail("CSR values must be finite");
+    const bool sliced_rows = sliced_rows_fit(nnz);
+    if (sliced_rows)
+        sliced::build(A.rows, A.off, A.idx, A.val, lens, rows_, sliced::elements_per_lane(nnz),
+                      stream);
 
     // transpose: stable sort of entry ids by column
     AMFLS_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (cols_ + 1), stream));
@@ -874,6 +895,9 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
         T.off, cols_, nnz, &w->err, &w->max_len_c, lens, elems_per_lane_, bins);
     AMFLS_LAUNCHED();
     build_bins(T, bins, stream);
+    if (sliced_rows)
+        sliced::build(T.rows, T.off, T.idx, T.val, lens, cols_, sliced::elements_per_lane(nnz),
+                      stream);
 
     // int32 offsets and tilings of both sides for the streamed products
     for (Side* sd : {&A, &T}) {
@@ -1059,6 +1083,16 @@ void CsrOperator::single_column_schedule(int chains[2], double microseconds[4]) 
         microseconds[2 * i] = sides[i]->tuned_us[0];
         microseconds[2 * i + 1] = sides[i]->tuned_us[1];
     }
+}
+
+bool CsrOperator::resident(ResidentOperator* view) const {
+    if (!a_->rows.tasks || !t_->rows.tasks) return false;
+    view->a = a_->rows.side;
+    view->t = t_->rows.side;
+    view->rows = rows_;
+    view->cols = cols_;
+    view->nonzeros = nnz_;
+    return true;
 }
 
 bool CsrOperator::product1(bool transpose, const double* x, const Epilogue& ep,

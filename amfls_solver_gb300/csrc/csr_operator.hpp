@@ -42,6 +42,7 @@ public:
                                  double* x_lo, int* finite, cudaStream_t s) const override;
     bool product1(bool transpose, const double* x, const Epilogue& ep,
                   cudaStream_t s) const override;
+    bool resident(ResidentOperator* view) const override;
     // Tiling of the single-column products per side (A, then the stored
     // transpose): 1 = chain groups, 0 = row blocks; the autotuner's timings
     // (microseconds per product, row blocks then chain groups, 0 = not timed).

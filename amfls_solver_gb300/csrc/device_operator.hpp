@@ -90,6 +90,8 @@ inline ValidationModel reduced_model(const ValidationModel& m, ValueType type) {
     return r;
 }
 
+struct ResidentOperator;
+
 class DeviceOperator {
 public:
     virtual ~DeviceOperator() = default;
@@ -118,6 +120,12 @@ public:
     virtual bool product1(bool transpose, const double* x, const Epilogue& ep,
                           cudaStream_t s) const {
         (void)transpose; (void)x; (void)ep; (void)s;
+        return false;
+    }
+    // The tables with which the resident level kernel computes the products
+    // itself; false when the operator has none.
+    virtual bool resident(ResidentOperator* view) const {
+        (void)view;
         return false;
     }
     // Storage kind for diagnostics: 0 CSR, 1 row-major dense, 2 column-major

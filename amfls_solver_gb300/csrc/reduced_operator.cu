@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "reduced_operator.hpp"
+#include "resident_levels.hpp"
 
 namespace amfls_gpu {
 namespace {
@@ -439,6 +440,13 @@ void AugmentedOperator::apply_transpose(const double* y, int block_cols, double*
                                                                 root_, x + c0 * n);
         AMFLS_LAUNCHED();
     }
+}
+
+bool AugmentedOperator::resident(ResidentOperator* view) const {
+    if (!a_.resident(view) || view->augmented) return false;
+    view->augmented = true;
+    view->root = root_;
+    return true;
 }
 
 bool AugmentedOperator::product1(bool transpose, const double* x, const Epilogue& ep,

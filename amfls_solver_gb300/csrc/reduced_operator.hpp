@@ -75,6 +75,7 @@ public:
     ValidationModel validation_error_model() const override { return model_; }
     bool product1(bool transpose, const double* x, const Epilogue& ep,
                   cudaStream_t s) const override;
+    bool resident(ResidentOperator* view) const override;
 
 private:
     const DeviceOperator& a_;

@@ -1,6 +1,9 @@
 // Device block Golub-Kahan workspace (see workspace.hpp for the layout).
 //
-// One width-one level (krylov_workspace.cpp:589-831) is the kernel chain
+// Width-one levels of CSR operators run in the resident level kernel
+// (resident_levels.cu).  For every other operator, for bases beyond
+// kResidentMaxBasis columns and with graphs switched off, one width-one level
+// (krylov_workspace.cpp:589-831) is the kernel chain
 //   begin        decide on the device whether the level runs (can_advance,
 //                depth target); reset the step audit
 //   A^T u        fused SpMV^T: r = A^T u - beta v_prev, ||A^T u||, ||r||
@@ -33,6 +36,7 @@
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "level_decisions.cuh"
 #include "vector_ops.hpp"
 #include "workspace.hpp"
 
@@ -76,7 +80,6 @@ void stream_wait(cudaStream_t stream) {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr double kEps = 2.220446049250313e-16;
 // V^T r by blocks (vt_r_kernel) launches about 16 blocks per SM (panels x
 // row chunks); kMaxGemvTargetBlocks bounds it for sizing the partials
 inline int gemv_target_blocks() { return 16 * sm_count(); }
@@ -96,136 +99,6 @@ bool use_warp_sweeps(long long n) {
     return n < kWarpSweepMaxRows;
 }
 
-enum Hook { kHookNone = 0, kHookRightPass1 = 1, kHookRightPass2 = 2 };
-
-__device__ inline bool dfinite(double v) { return isfinite(v); }
-
-// Rank decision for the width-one right residual (krylov_workspace.cpp:197-310,
-// scalar branch) after its final projection pass.
-__device__ void decide_right(DevState* st, int m, int n) {
-    const double scale = st->right_scale;
-    const double after = st->norm_after;
-    const int k = st->k;
-    const int dim = max(max(1, m), max(n, max(k, 1)));
-    const double cutoff = (scale >= 0.0 && dfinite(scale)) ? 64.0 * kEps * dim * scale
-                                                           : __builtin_huge_val();
-    const bool finite = dfinite(scale) && dfinite(after) && !st->coeff_nonfinite;
-    const int max_rank = min(1, st->basis_limit - k);  // combined width is one
-    StepAudit& a = st->audit;
-    int rank = 0;
-    double discarded = after, tracked = 0.0;
-    bool positive = false;
-    if (!finite) {
-        discarded = __builtin_huge_val();
-        tracked = __builtin_huge_val();  // tracked prefix = active width = 1
-    } else if (max_rank == 0) {
-        tracked = after;
-    } else if (after > cutoff) {
-        rank = 1;
-        discarded = 0.0;
-    } else if (after > 0.0) {
-        positive = true;
-        tracked = after;
-    }
-    a.retained_right_width = rank;
-    a.right_rank_cutoff = cutoff;
-    a.right_discarded_residual_norm = discarded;
-    a.right_active_discarded_residual_norm = tracked;
-    a.right_positive_finite_below_cutoff = positive;
-    a.right_nonfinite_residual = !finite;
-    a.right_rank_loss = rank < max_rank;
-    a.right_basis_cap_truncation = max_rank < 1;
-    const bool truncated = a.right_rank_loss && positive && tracked > 0.0;
-    if (truncated || !finite) st->reliable = 0;
-    st->right_rank = rank;
-    if (rank == 0) {
-        st->left_width = 0;
-        st->active_first = st->rows_t;
-        st->prev_right_first = k;
-        st->prev_right_width = 0;
-        st->coupling = 0.0;
-        st->level_ok = 0;
-        st->go = 0;
-        return;
-    }
-    st->right_factor = after;
-    st->inv_right = 1.0 / after;
-    st->search_a_calls += 1;
-    st->search_a_columns += 1;
-}
-
-// Rank decision of the left residual and the T / g update
-// (krylov_workspace.cpp:736-830).
-__device__ void decide_left(DevState* st, int m, int n, double* alpha, double* beta, double* g) {
-    const double scale = st->left_scale;
-    const double after = st->left_norm;
-    const int dim = max(max(1, m), n);
-    const double cutoff = (scale >= 0.0 && dfinite(scale)) ? 64.0 * kEps * dim * scale
-                                                           : __builtin_huge_val();
-    const bool finite = dfinite(scale) && dfinite(after) && dfinite(st->left_coeff);
-    const int old_left = st->rows_t;
-    const int max_rank = min(min(1, m - old_left), st->basis_limit + 1 - old_left);
-    StepAudit& a = st->audit;
-    int rank = 0;
-    double discarded = after;
-    bool positive = false;
-    if (!finite) {
-        discarded = __builtin_huge_val();
-    } else if (max_rank <= 0) {
-        // nothing retained, nothing tracked
-    } else if (after > cutoff) {
-        rank = 1;
-        discarded = 0.0;
-    } else if (after > 0.0) {
-        positive = true;
-    }
-    a.retained_next_left_width = rank;
-    a.left_rank_cutoff = cutoff;
-    a.left_discarded_residual_norm = discarded;
-    a.left_positive_finite_below_cutoff = positive;
-    a.left_nonfinite_residual = !finite;
-    a.left_rank_loss = rank < max_rank;
-    a.left_basis_cap_truncation = max_rank < 1;
-    const bool truncated = (a.left_rank_loss && positive);
-    if (truncated || !finite) st->reliable = 0;
-    if (!finite) {
-        st->level_ok = 0;
-        st->go = 0;
-        return;
-    }
-    const int k_old = st->k;
-    alpha[k_old] = st->right_factor + st->left_coeff;  // active coupling + coefficient
-    beta[k_old] = rank ? after : 0.0;
-    if (rank) {
-        st->inv_left = 1.0 / after;
-        g[old_left] = st->b_dot * st->inv_left;
-    }
-    st->left_rank = rank;
-    st->k = k_old + 1;
-    st->active_first = old_left;
-    st->rows_t = old_left + rank;
-    st->left_width = rank;
-    st->prev_right_first = k_old;
-    st->prev_right_width = 1;
-    st->coupling = after;
-    st->depth += 1;
-    st->level_ok = 1;
-    st->levels_run += 1;
-    a.basis_rank_after = k_old + 1;
-    if (!rank) st->go = 0;  // nothing to normalise; the process stops here
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ bool can_advance_dev(const DevState* st) {
-    return st->reliable && (st->left_width + st->pending > 0) && st->k < st->basis_limit &&
-           st->depth < st->target_depth;
-}
-
 __global__ void set_target_kernel(DevState* st, int target_depth, int iterations) {
     if (threadIdx.x != 0) return;
     st->target_depth = target_depth;
@@ -233,29 +106,7 @@ __global__ void set_target_kernel(DevState* st, int target_depth, int iterations
 }
 
 __global__ void level_begin_kernel(DevState* st) {
-    if (threadIdx.x != 0) return;
-    st->body_runs += 1;
-    const bool go = can_advance_dev(st) && st->iterations_left > 0;
-    st->iterations_left -= 1;
-    st->go = go ? 1 : 0;
-    if (!go) return;
-    st->sub_col = st->prev_right_width > 0 ? st->prev_right_first : 0;
-    st->t_mark = global_ns();
-    StepAudit a;
-    memset(&a, 0, sizeof(a));
-    a.left_input_width = st->left_width + st->pending;
-    a.basis_rank_before = st->k;
-    a.basis_rank_after = st->k;
-    st->audit = a;
-    st->coupling_eff = (st->prev_right_width > 0 && st->left_width > 0) ? st->coupling : 0.0;
-    st->second_pass = 0;
-    st->right_rank = 0;
-    st->left_rank = 0;
-    st->coeff_nonfinite = 0;
-    st->sweep_fp64 = 0;
-    st->level_ok = 0;
-    st->search_at_calls += 1;
-    st->search_at_columns += st->left_width + st->pending;
+    if (threadIdx.x == 0) begin_level(st);
 }
 
 // after A^T u: scale and norm_before from the fused reduction
@@ -473,47 +324,6 @@ v_c_kernel(double* const* __restrict__ panels, int n, int k_arg, const double* _
 // amplified by about cond(A), so a single solve of an ill-conditioned
 // problem to FP64 accuracy stalls on it (the certificate then reports the
 // failure; it never certifies a wrong x).
-constexpr double kReducedCoeffBound = 1e-3;
-
-// Storage of the basis copy: FP32, or FP16 holding 2^8 v (the entries of a
-// unit vector then stay in FP16's normal range down to 2.4e-7; products and
-// sums run in FP32 and the results are scaled back by 2^-8, exactly).
-template <typename S>
-struct RedStore;
-// kFlushSteps: steps (of 4 rows per lane) summed in FP32 before a lane's
-// partial sums go into FP64.  Each fold costs FP64 instructions (this GPU
-// retires two FP64 lanes per SM clock), which an FP16 copy, reading half the
-// bytes per element, must amortise over more rows; its own rounding (2^-11)
-// dwarfs the longer FP32 sums' (64 terms: about 2^-18).
-template <>
-struct RedStore<float> {
-    static constexpr int kFlushSteps = 4;
-    static constexpr float kInvScale = 1.0f;
-    __device__ static void load8(const float* p, float v[8]) {
-        const float4 a = __ldcs(reinterpret_cast<const float4*>(p));
-        const float4 b = __ldcs(reinterpret_cast<const float4*>(p) + 1);
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    }
-    __device__ static float store(double v) { return __double2float_rn(v); }
-};
-template <>
-struct RedStore<__half> {
-    static constexpr int kFlushSteps = 16;
-    static constexpr float kInvScale = 1.0f / 256.0f;
-    __device__ static void load8(const __half* p, float v[8]) {
-        const uint4 u = __ldcs(reinterpret_cast<const uint4*>(p));
-        const __half2* h = reinterpret_cast<const __half2*>(&u);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 f = __half22float2(h[i]);
-            v[2 * i] = f.x;
-            v[2 * i + 1] = f.y;
-        }
-    }
-    __device__ static __half store(double v) { return __float2half_rn(__double2float_rn(v * 256.0)); }
-};
-
 // r~ = fl32(r) for the reduced pass (only when the level projects).
 __global__ void round_residual_kernel(const double* __restrict__ r, float* __restrict__ r32, int n,
                                       const DevState* st) {
@@ -888,20 +698,6 @@ sweep_vt_kernel(double* const* __restrict__ panels, int n, const double* __restr
     }
 }
 
-// The DGKS test and rank decision after the right residual's norm is known
-// (the hooks of v_c_kernel).
-__device__ inline void finish_right_norm(DevState* st, int hook, double sumsq, int m, int n) {
-    st->norm_after = sqrt(sumsq);
-    if (hook == kHookRightPass1) {
-        const double before = st->norm_before, after = st->norm_after;
-        const bool again = isfinite(before) && isfinite(after) && after < 0.70710678118654757 * before;
-        st->second_pass = again ? 1 : 0;
-        if (!again) decide_right(st, m, n);
-    } else if (hook == kHookRightPass2) {
-        decide_right(st, m, n);
-    }
-}
-
 // out = r_in - V c (subtract) or V c over the current basis, its sum of
 // squares, then `hook`.
 __global__ void __launch_bounds__(kThreads)
@@ -1241,7 +1037,7 @@ template class PanelStoreT<__half>;
 
 Workspace::Workspace(const DeviceOperator& op, const double* d_b, double regularization,
                      int maximum_basis_size, cudaStream_t stream, bool time_operators,
-                     bool use_graphs, int reduced_basis)
+                     bool use_graphs, int reduced_basis, int resident_sms)
     : op_(op), stream_(stream), m_(op.rows()), n_(op.cols()), reg_(regularization),
       time_ops_(time_operators), use_graphs_(use_graphs), b_(d_b) {
     if (m_ <= 0 || n_ <= 0) throw std::invalid_argument("block Golub-Kahan operator dimensions must be positive");
@@ -1303,6 +1099,15 @@ Workspace::Workspace(const DeviceOperator& op, const double* d_b, double regular
             AMFLS_CUDA(cudaMemsetAsync(red_tickets_, 0, sizeof(unsigned) * (max_panels + 1),
                                        stream_));
         }
+        if (resident_sms > 0 && op_.resident(&resident_op_)) {
+            resident_grid_ = std::min(resident_sms, sm_count());
+            stream_alloc(&resident_red_, sizeof(double) * resident_red_doubles(resident_grid_),
+                         stream_);
+            stream_alloc(&resident_part_,
+                         sizeof(double) * resident_part_doubles(resident_grid_, max_panels),
+                         stream_);
+            stream_alloc(&resident_barrier_, sizeof(unsigned), stream_);
+        }
         AMFLS_CUDA(cudaStreamCreateWithFlags(&capture_stream_, cudaStreamNonBlocking));
         std::memset(&host_, 0, sizeof(host_));
         host_.reliable = 1;
@@ -1320,6 +1125,10 @@ Workspace::~Workspace() { release(); }
 
 void Workspace::release() noexcept {
     cudaStreamSynchronize(stream_);
+    lease_.release();
+    stream_free(resident_red_, stream_);
+    stream_free(resident_part_, stream_);
+    stream_free(resident_barrier_, stream_);
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     if (graph_) cudaGraphDestroy(graph_);
     if (capture_stream_) cudaStreamDestroy(capture_stream_);
@@ -1628,6 +1437,11 @@ void Workspace::advance_to(int target_depth) {
     V_->ensure_columns(host_.k + levels + 1);
     if (V32_) V32_->ensure_columns(host_.k + levels + 1);
     if (V16_) V16_->ensure_columns(host_.k + levels + 1);
+    interval_graph_ = false;
+    if (resident_grid_ > 0 && host_.k + levels <= kResidentMaxBasis) {
+        run_resident(levels, target_depth);
+        return;
+    }
     const int pneed = (host_.k + levels + 31) / 32;
     int pcap = 4;
     while (pcap < pneed) pcap *= 2;
@@ -1640,6 +1454,38 @@ void Workspace::advance_to(int target_depth) {
     if (!graph_exec_ || pcap > graph_pcap_) build_graph(pcap);
     AMFLS_CUDA(cudaGraphLaunch(graph_exec_, stream_));
     ++graph_launches_;
+    interval_graph_ = true;
+}
+
+void Workspace::run_resident(int levels, int target_depth) {
+    ResidentArgs a{};
+    a.st = dstate_;
+    a.a = resident_op_.a;
+    a.t = resident_op_.t;
+    a.m = resident_op_.rows;
+    a.ml = m_;
+    a.n = n_;
+    a.root = resident_op_.root;
+    a.b = b_;
+    a.u = U_;
+    a.y = Y_;
+    a.r = R_;
+    a.v = vnew_;
+    a.panels = V_->device_table();
+    a.npanels = (host_.k + levels + 31) / 32;
+    if (V16_) a.shadow = reinterpret_cast<void* const*>(V16_->device_table());
+    else if (V32_) a.shadow = reinterpret_cast<void* const*>(V32_->device_table());
+    a.alpha = alpha_;
+    a.beta = beta_;
+    a.g = g_;
+    a.red = resident_red_;
+    a.part = resident_part_;
+    a.barrier = resident_barrier_;
+    lease_.acquire(resident_grid_);
+    AMFLS_CUDA(cudaMemsetAsync(resident_barrier_, 0, sizeof(unsigned), stream_));
+    set_target_kernel<<<1, 32, 0, stream_>>>(dstate_, target_depth, levels);
+    AMFLS_LAUNCHED();
+    launch_resident_levels(a, resident_grid_, host_.k + levels, reduced_storage_, stream_);
 }
 
 bool Workspace::advance_level() {
@@ -1654,7 +1500,10 @@ bool Workspace::advance_level() {
 void Workspace::sync() {
     AMFLS_CUDA(cudaMemcpyAsync(&host_, dstate_, sizeof(DevState), cudaMemcpyDeviceToHost, stream_));
     stream_wait(stream_);
-    if (use_graphs_) {  // kernels the device ran inside graph-launched intervals
+    lease_.release();
+    if (host_.barrier_timeout)
+        throw std::runtime_error("resident level kernel: a grid barrier timed out");
+    if (interval_graph_) {  // kernels the device ran inside graph-launched intervals
         launch_count() += body_kernels_ * (host_.body_runs - counted_body_runs_);
     }
     counted_body_runs_ = host_.body_runs;

@@ -11,10 +11,10 @@
 //      as in the reference); P pending P*Omega, m x p.
 //   T  projected operator: lower bidiagonal at width one, kept as the two
 //      diagonals alpha_j = T(j, j), beta_{j+1} = T(j+1, j); g = U^T b.
-// Width-one levels run entirely on the device (DevState decisions): one level
-// is captured as the body of a CUDA graph WHILE node, so a whole checkpoint
-// interval is a single graph launch.  Wider blocks use the host-synchronised
-// block path.
+// Width-one levels run entirely on the device (DevState decisions): a whole
+// checkpoint interval is one launch, of the resident level kernel for CSR
+// operators, else of a CUDA graph whose WHILE node runs one captured level
+// after the other.  Wider blocks use the host-synchronised block path.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "device_operator.hpp"
+#include "resident_levels.hpp"
 #include "vector_ops.hpp"
 #include "workspace_state.hpp"
 
@@ -62,10 +63,11 @@ class Workspace {
 public:
     // reduced_basis (a ReducedStorage): width-one levels keep an FP32 or FP16
     // copy of V and run their first projection pass on it (see
-    // enqueue_level_kernels).
+    // enqueue_level_kernels).  resident_sms: SMs the resident level kernel may
+    // take (0: none, the kernel chain runs the levels).
     Workspace(const DeviceOperator& op, const double* d_b, double regularization,
               int maximum_basis_size, cudaStream_t stream, bool time_operators,
-              bool use_graphs = true, int reduced_basis = kReducedOff);
+              bool use_graphs = true, int reduced_basis = kReducedOff, int resident_sms = 0);
     ~Workspace();
     Workspace(const Workspace&) = delete;
     Workspace& operator=(const Workspace&) = delete;
@@ -120,6 +122,7 @@ private:
     // (the destructor, and a constructor that fails after allocating)
     void release() noexcept;
     void enqueue_level_kernels(cudaStream_t s, int pcap);
+    void run_resident(int levels, int target_depth);
     void build_graph(int pcap);
     void invalidate_graph();
     void ensure_t_capacity(int cols);
@@ -221,6 +224,15 @@ private:
     long long body_kernels_ = 0;       // kernels in the captured level body
     long long counted_body_runs_ = 0;  // body runs already added to launch_count()
     long long graph_launches_ = 0;
+    bool interval_graph_ = false;      // the last interval ran as a graph
+    // resident level kernel: the operator's tables, its grid, the SMs it
+    // holds between a launch and the sync() that ends the interval
+    ResidentOperator resident_op_;
+    int resident_grid_ = 0;
+    SmLease lease_;
+    double* resident_red_ = nullptr;
+    double* resident_part_ = nullptr;
+    unsigned* resident_barrier_ = nullptr;
     unsigned long long seen_a_ns_ = 0, seen_at_ns_ = 0;
 
     // block mode state (host side; device buffers below)

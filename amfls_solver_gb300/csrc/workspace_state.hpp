@@ -59,6 +59,7 @@ struct DevState {
     int iterations_left;  // hard cap on loop iterations of the enqueued run
     int sub_col;          // V column subtracted by the coupling (0 when none)
     int sweep_fp64;       // reduced-basis level: redo the projection in FP64
+    int barrier_timeout;  // a grid barrier of the resident kernel gave up waiting
     // device time of search operator calls (globaltimer, ns)
     unsigned long long a_ns;
     unsigned long long at_ns;
