@@ -52,9 +52,9 @@ class Run {
 public:
     Run(const DeviceOperator& op, cudaStream_t s) : op_(op), s_(s) {
         stream_alloc(&partials_, sizeof(double) * 2 * kMaxVectors * kMaxGridCap, s_);
-        stream_alloc(&counter_, sizeof(unsigned), s_);
+        stream_alloc(&counter_, sizeof(unsigned) * kMaxVectors, s_);  // a ticket per vector
         stream_alloc(&norms_, sizeof(NormResult), s_);
-        AMFLS_CUDA(cudaMemsetAsync(counter_, 0, sizeof(unsigned), s_));
+        AMFLS_CUDA(cudaMemsetAsync(counter_, 0, sizeof(unsigned) * kMaxVectors, s_));
         for (auto& e : ev_) AMFLS_CUDA(cudaEventCreate(&e));
     }
     ~Run() {
@@ -100,8 +100,7 @@ public:
         }
         norm_passes(set, norms_, partials_, counter_, s_);
         NormResult h{};
-        AMFLS_CUDA(cudaMemcpyAsync(&h, norms_, sizeof(NormResult), cudaMemcpyDeviceToHost, s_));
-        stream_wait(s_);
+        read_back(&h, norms_, s_);
         settle();
         return h;
     }

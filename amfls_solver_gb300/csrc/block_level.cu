@@ -85,8 +85,7 @@ double Workspace::device_norm(const double* x, long long count) {
     set.count = 1;
     norm_passes(set, dnorm_, partials_, counter_ + 1, stream_);
     NormResult h{};
-    AMFLS_CUDA(cudaMemcpyAsync(&h, dnorm_, sizeof(NormResult), cudaMemcpyDeviceToHost, stream_));
-    stream_wait(stream_);
+    read_back(&h, dnorm_, stream_);
     return euclid_from(h, 0);
 }
 

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstring>
 #include <stdexcept>
 #include <string>
 
@@ -54,11 +55,29 @@ inline void stream_free(const void* p, cudaStream_t s) {
 // buffers.  Called by each solve; takes effect once per device.
 void keep_pool_memory();
 
-// Waits until the work enqueued on `stream` so far has finished, blocking the
-// calling thread on a blocking-sync event instead of spinning (concurrent
-// solves on many host threads then leave the CPU cores to the threads that
-// launch work).
+// Waits until the work enqueued on `stream` so far has finished: polls for a
+// few tens of microseconds (short waits then end without a thread wake-up),
+// then blocks the calling thread on a blocking-sync event (concurrent solves
+// on many host threads leave the CPU cores to the threads that launch work).
 void stream_wait(cudaStream_t stream);
+
+// A page of pinned host memory of the calling thread, freed with the thread:
+// the landing place of the small device-to-host reads of a solve.  The first
+// half belongs to state that is read and used at once, the second half to
+// the projected solve's flags (read after the next wait).
+constexpr size_t kPinnedBytes = 8192;
+unsigned char* pinned_page();
+
+// Copies a small device object to the host and waits for it.
+template <typename T>
+inline void read_back(T* host, const T* device, cudaStream_t stream) {
+    static_assert(sizeof(T) <= kPinnedBytes / 2);
+    unsigned char* page = pinned_page();
+    check_cuda(cudaMemcpyAsync(page, device, sizeof(T), cudaMemcpyDeviceToHost, stream),
+               "cudaMemcpyAsync");
+    stream_wait(stream);
+    std::memcpy(host, page, sizeof(T));
+}
 
 // Streaming multiprocessors of the current device
 // (cudaDevAttrMultiProcessorCount), queried once per device.

@@ -379,20 +379,26 @@ public:
               Statistics& stats, cudaStream_t stream)
         : ws_(ws), validator_(op, d_b, reg, stream), stats_(stats), stream_(stream), n_(op.cols()) {
         for (auto& p : buf_) stream_alloc(&p, sizeof(double) * std::max(1, n_), stream_);
+        for (auto& e : projected_) AMFLS_CUDA(cudaEventCreate(&e));
     }
     ~Evaluator() {
         cudaStreamSynchronize(stream_);
+        for (auto e : projected_)
+            if (e) cudaEventDestroy(e);
         for (auto p : buf_) stream_free(p, stream_);
     }
 
     Candidate evaluate(double tol, int epoch, int aux, int keep_a, int keep_b, TraceRow* row) {
         int slot = 0;
         while (slot == keep_a || slot == keep_b) ++slot;
-        const auto t0 = Clock::now();
+        AMFLS_CUDA(cudaEventRecord(projected_[0], stream_));
         ws_.solve_projected(buf_[slot]);
+        AMFLS_CUDA(cudaEventRecord(projected_[1], stream_));
+        const ValidationOutput v = validator_.validate(buf_[slot], tol);  // waits
+        float ms = 0.0f;
+        AMFLS_CUDA(cudaEventElapsedTime(&ms, projected_[0], projected_[1]));
+        stats_.projected_solve_seconds += ms * 1e-3;
         if (ws_.projected_flags() & 2) ++stats_.projected_rank_flags;
-        stats_.projected_solve_seconds += seconds_since(t0);
-        const ValidationOutput v = validator_.validate(buf_[slot], tol);
         Statistics& s = stats_;
         account_validation(s, v);
         Candidate c;
@@ -415,6 +421,7 @@ private:
     cudaStream_t stream_;
     int n_;
     double* buf_[3] = {nullptr, nullptr, nullptr};
+    cudaEvent_t projected_[2] = {};
 };
 
 // Fold the device counters of executed search levels into the statistics.

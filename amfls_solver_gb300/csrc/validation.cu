@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "dd.cuh"
+#include "epilogue.cuh"
 #include "fp_bounds.cuh"
 #include "validation.hpp"
 #include "vector_ops.hpp"
@@ -40,6 +41,13 @@ struct Model {
     long long apply_steps, transpose_steps;
 };
 
+// One pass over a vector: largest magnitude, plain sum of squares, and whether
+// a value is not finite.
+struct VectorStats {
+    double max_abs, sumsq;
+    int nonfinite, pad;
+};
+
 struct ValState {
     ValidationOutput out;
     Envelope env;
@@ -54,6 +62,11 @@ struct ValState {
     double corr_gnorm;
     double corr_step;
     double corr_hn_upper, corr_dn_upper, corr_adn_upper, corr_ad_err, corr_herr;
+    // one-wait path (base_fused_kernel and on)
+    int general;  // magnitudes beyond its range: the general path decides
+    int ran_correction_a, ran_correction_at;
+    RedResult ax, at, ad, h;  // sums the products came with
+    VectorStats x, d, q;
 };
 
 enum { ST_SUCCESS = 0, ST_WORK = 1, ST_BREAKDOWN = 4 };
@@ -188,6 +201,21 @@ __device__ void nominal_contract(ValidationOutput& r, double bnorm, double reg, 
     else r.stop_reason = SR_DEPTH;
 }
 
+// Status and stop reason from the certified bounds.
+__device__ void set_outcome(ValidationOutput& r, const Envelope& e, double reg, double tol) {
+    const bool passed = e.grad_upper == 0.0 ||
+                        (reg > 0.0 ? r.relative_energy_error_upper_bound <= tol
+                                   : r.backward_error_upper_bound <= tol);
+    r.status = passed ? ST_SUCCESS : ST_WORK;
+    if (e.grad_upper == 0.0) r.stop_reason = SR_EXACT;
+    else if (passed && reg > 0.0) r.stop_reason = SR_ENERGY;
+    else if (passed && r.compatible_backward_error_upper_bound <=
+                           r.least_squares_backward_error_upper_bound)
+        r.stop_reason = SR_COMPAT;
+    else if (passed) r.stop_reason = SR_LS;
+    else r.stop_reason = SR_DEPTH;
+}
+
 __device__ void certified_contract(ValidationOutput& r, const Envelope& e, double reg, double tol,
                                    bool has_ridge, double ridge_bound) {
     if (!e.certified) {
@@ -233,17 +261,7 @@ __device__ void certified_contract(ValidationOutput& r, const Envelope& e, doubl
         r.energy_error_upper_bound = r.relative_energy_error_upper_bound = kInf;
         r.objective_gap_upper_bound = kInf;
     }
-    const bool passed = e.grad_upper == 0.0 ||
-                        (reg > 0.0 ? r.relative_energy_error_upper_bound <= tol
-                                   : r.backward_error_upper_bound <= tol);
-    r.status = passed ? ST_SUCCESS : ST_WORK;
-    if (e.grad_upper == 0.0) r.stop_reason = SR_EXACT;
-    else if (passed && reg > 0.0) r.stop_reason = SR_ENERGY;
-    else if (passed && r.compatible_backward_error_upper_bound <=
-                           r.least_squares_backward_error_upper_bound)
-        r.stop_reason = SR_COMPAT;
-    else if (passed) r.stop_reason = SR_LS;
-    else r.stop_reason = SR_DEPTH;
+    set_outcome(r, e, reg, tol);
 }
 
 // nr slots: 0 b, 1 x, 2 Ax, 3 r, 4 A^T r, 5 g
@@ -384,8 +402,7 @@ __global__ void refined_contract_kernel(ValState* vs, Model mdl, long long m, lo
     certified_contract(r, e, reg, tol, false, 0.0);
 }
 
-__global__ void ridge_prelim_kernel(ValState* vs, double reg) {
-    if (threadIdx.x != 0) return;
+__device__ void ridge_prelim(ValState* vs, double reg) {
     ValidationOutput& r = vs->out;
     const Envelope& e = vs->env;
     vs->need_correction = 0;
@@ -406,6 +423,40 @@ __global__ void ridge_prelim_kernel(ValState* vs, double reg) {
         vs->corr_gnorm = gn;
         vs->need_correction = 1;
     }
+}
+
+__global__ void ridge_prelim_kernel(ValState* vs, double reg) {
+    if (threadIdx.x == 0) ridge_prelim(vs, reg);
+}
+
+// Stage 2 of the correction: the corrected energy bound from q (slot 3).
+__device__ void correction_bound(ValState* vs, const NormResult& nr, long long n, double reg) {
+    ValidationOutput& r = vs->out;
+    const Interval qn = nint(nr, 3);
+    const double step = vs->corr_step;
+    const double curv = vs->dot;
+    const double axpy_err = one_op_radius(qn.upper, vs->corr_gnorm > 0.0 && vs->corr_hn_upper > 0.0,
+                                          n, fpb::kUnitRoundoff);
+    const double q_err =
+        fpb::up_add(fpb::up_add(vs->env.grad_radius, fpb::up_mul(step, vs->corr_herr)), axpy_err);
+    const double q_up = fpb::up_add(qn.upper, q_err);
+    const double ad_true = fpb::up_add(vs->corr_adn_upper, vs->corr_ad_err);
+    const double step2 = fpb::up_mul(step, step);
+    const double dn = vs->corr_dn_upper;
+    const double de2 = fpb::up_add(fpb::up_mul(ad_true, ad_true), fpb::up_mul(reg, fpb::up_mul(dn, dn)));
+    const double zhz = fpb::up_mul(step2, de2);
+    const double two_cross = fpb::up_mul(2.0, fpb::up_mul(step, fpb::up_mul(dn, q_up)));
+    const double qsq = fpb::up_mul(q_up, q_up);
+    const double corrected =
+        fpb::up_sqrt(fpb::up_add(zhz, fpb::up_add(two_cross, fpb::up_div(qsq, reg))));
+    vs->need_correction = 0;
+    if (isnan(corrected)) return;
+    r.ridge_corrected_energy_error_upper_bound = corrected;
+    r.ridge_correction_gamma = 1.0 / curv;
+    r.ridge_correction_z_h_z = zhz;
+    r.ridge_correction_two_abs_z_t_q = two_cross;
+    r.ridge_correction_q_norm_squared = qsq;
+    r.ridge_correction_disposition = RC_NOT_IMPROVED;
 }
 
 // correction stage scalars; nr2 slots: 0 d, 1 Ad, 2 h, 3 q
@@ -466,31 +517,7 @@ __global__ void correction_step_kernel(ValState* vs, Model mdl, long long m, lon
         vs->need_correction = 0;
         return;
     }
-    const Interval qn = nint(nr, 3);
-    const double step = vs->corr_step;
-    const double curv = vs->dot;
-    const double axpy_err = one_op_radius(qn.upper, vs->corr_gnorm > 0.0 && vs->corr_hn_upper > 0.0,
-                                          n, fpb::kUnitRoundoff);
-    const double q_err =
-        fpb::up_add(fpb::up_add(vs->env.grad_radius, fpb::up_mul(step, vs->corr_herr)), axpy_err);
-    const double q_up = fpb::up_add(qn.upper, q_err);
-    const double ad_true = fpb::up_add(vs->corr_adn_upper, vs->corr_ad_err);
-    const double step2 = fpb::up_mul(step, step);
-    const double dn = vs->corr_dn_upper;
-    const double de2 = fpb::up_add(fpb::up_mul(ad_true, ad_true), fpb::up_mul(reg, fpb::up_mul(dn, dn)));
-    const double zhz = fpb::up_mul(step2, de2);
-    const double two_cross = fpb::up_mul(2.0, fpb::up_mul(step, fpb::up_mul(dn, q_up)));
-    const double qsq = fpb::up_mul(q_up, q_up);
-    const double corrected =
-        fpb::up_sqrt(fpb::up_add(zhz, fpb::up_add(two_cross, fpb::up_div(qsq, reg))));
-    vs->need_correction = 0;
-    if (isnan(corrected)) return;
-    r.ridge_corrected_energy_error_upper_bound = corrected;
-    r.ridge_correction_gamma = 1.0 / curv;
-    r.ridge_correction_z_h_z = zhz;
-    r.ridge_correction_two_abs_z_t_q = two_cross;
-    r.ridge_correction_q_norm_squared = qsq;
-    r.ridge_correction_disposition = RC_NOT_IMPROVED;
+    correction_bound(vs, nr, n, reg);
 }
 
 __global__ void finish_kernel(ValState* vs, double reg, double tol) {
@@ -584,6 +611,385 @@ __global__ void correction_q_kernel(const double* h, const double* g, const ValS
         q[i] = fma(-step, h[i], g[i]);
 }
 
+// ---------------------------------------------- validation with one wait ----
+//
+// The products' epilogues already sum what the contracts need, so the base
+// pair takes one more pass (over x) and no norm kernels, the ridge correction
+// runs behind a device flag, and the host waits once per candidate.  The
+// scalar envelope is some hundred dependent FP64 operations, divisions and
+// square roots among them, at 64 clocks or more each; its independent parts run
+// in the lanes of a warp or in different warps (each SM quarter has its own
+// FP64 unit).  2000 x 500, one candidate: 0.55 -> 0.2 ms.
+//
+// A plain sum of squares stands in for the scaled one while every largest
+// magnitude lies in kPlainLow .. kPlainHigh: powers of two scale exactly, so
+// the bounds are those of norm_interval with exponent 0, and what underflows
+// is below the denormal term they already carry.  Other candidates (and values
+// that are not finite) take the general path.
+constexpr double kPlainLow = 0x1p-300, kPlainHigh = 0x1p300;
+constexpr int kContractThreads = 128;
+
+__device__ __forceinline__ bool plain_range(double mx) {
+    return mx == 0.0 || (mx > kPlainLow && mx < kPlainHigh);
+}
+
+// Adds a thread's values to a vector's statistics; the last block writes them.
+// Returns true in that block.  partials: 3 per block.
+__device__ inline bool finish_stats(double sumsq, unsigned long long mx, int bad, double* partials,
+                                    unsigned* ticket, VectorStats* out) {
+    __shared__ double red[32];
+    __shared__ unsigned long long ured[32];
+    double sq = block_sum(sumsq, red);
+    unsigned long long m = block_umax(mx, ured);
+    const int any = __syncthreads_or(bad);
+    if (threadIdx.x == 0) {
+        partials[3 * blockIdx.x] = sq;
+        partials[3 * blockIdx.x + 1] = __longlong_as_double((long long)m);
+        partials[3 * blockIdx.x + 2] = any ? 1.0 : 0.0;
+    }
+    if (!arrive_last(ticket, gridDim.x)) return false;
+    sq = 0.0;
+    m = 0;
+    bad = 0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+        sq += partials[3 * b];
+        const unsigned long long v = __double_as_longlong(partials[3 * b + 1]);
+        m = v > m ? v : m;
+        if (partials[3 * b + 2] != 0.0) bad = 1;
+    }
+    sq = block_sum(sq, red);
+    m = block_umax(m, ured);
+    const int all = __syncthreads_or(bad);
+    if (threadIdx.x == 0) {
+        out->sumsq = sq;
+        out->max_abs = __longlong_as_double((long long)m);
+        out->nonfinite = all;
+    }
+    __syncthreads();
+    return true;
+}
+
+__device__ __forceinline__ void add_stats(double v, double& sumsq, unsigned long long& mx,
+                                          int& bad) {
+    sumsq = fma(v, v, sumsq);
+    const unsigned long long a = __double_as_longlong(v) & 0x7fffffffffffffffull;
+    if (a >= 0x7ff0000000000000ull) bad = 1;
+    else if (a > mx) mx = a;
+}
+
+__global__ void stats_kernel(const double* x, long long n, double* partials, unsigned* ticket,
+                             VectorStats* out) {
+    double sq = 0.0;
+    unsigned long long mx = 0;
+    int bad = 0;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x)
+        add_stats(x[i], sq, mx, bad);
+    finish_stats(sq, mx, bad, partials, ticket, out);
+}
+
+__device__ void set_norm(NormResult& nr, int i, double mx, double sumsq, long long count) {
+    nr.max_abs[i] = mx;
+    nr.scaled_sumsq[i] = sumsq;
+    nr.exponent[i] = 0;
+    nr.nonfinite[i] = 0;
+    nr.count[i] = count;
+}
+
+// certified_contract for a whole block: square roots and quotients side by side.
+__device__ void certified_contract_block(ValidationOutput& r, const Envelope& e, double reg,
+                                         double tol, bool has_ridge, double ridge_bound) {
+    __shared__ double root[4], quot[4];
+    const int t = threadIdx.x;
+    const double opl = r.operator_norm_lower_bound;
+    if (!e.certified) {
+        if (t == 0) certified_contract(r, e, reg, tol, has_ridge, ridge_bound);
+        __syncthreads();
+        return;
+    }
+    // augmented residual norm (0: lower, 1: upper), operator norm, sqrt(reg)
+    if (t < 4) {
+        double v;
+        if (t == 1) v = fpb::up_add(fpb::up_mul(e.res_upper, e.res_upper),
+                                    fpb::up_mul(reg, fpb::up_mul(e.sol_upper, e.sol_upper)));
+        else if (t == 0) v = fpb::down_add(fpb::down_mul(e.res_lower, e.res_lower),
+                                           fpb::down_mul(reg, fpb::down_mul(e.sol_lower, e.sol_lower)));
+        else v = t == 2 ? fpb::down_add(fpb::down_mul(opl, opl), reg) : reg;
+        root[t] = t == 1 ? fpb::up_sqrt(v) : fpb::down_sqrt(v);
+    }
+    __syncthreads();
+    const double aopl = root[2];
+    if (t < 4) {
+        double num = e.grad_upper, den;
+        if (t == 0) {
+            num = root[1];
+            den = fpb::down_add(fpb::down_mul(aopl, e.sol_lower), e.b_lower);
+        } else if (t == 1) {
+            den = fpb::down_mul(aopl, root[0]);
+        } else if (t == 2) {
+            den = fpb::down_add(fpb::down_mul(fpb::down_add(fpb::down_mul(opl, opl), reg), e.sol_lower),
+                                fpb::down_mul(opl, e.b_lower));
+        } else {
+            den = root[3];
+        }
+        quot[t] = fpb::up_div(num, den);
+    }
+    __syncthreads();
+    if (t == 0) {
+        r.augmented_operator_norm_lower_bound = aopl;
+        r.compatible_backward_error_upper_bound = quot[0];
+        r.least_squares_backward_error_upper_bound = quot[1];
+        r.backward_error_upper_bound = fmin(quot[0], quot[1]);
+        r.relative_normal_residual_upper_bound = quot[2];
+        if (reg > 0.0) {
+            const double err = has_ridge ? ridge_bound : quot[3];
+            r.energy_error_upper_bound = err;
+            r.objective_gap_upper_bound = fpb::up_mul(err, err);
+            r.relative_energy_error_upper_bound =
+                fpb::up_div(err, fpb::down_diff(e.energy_lower, err));
+        } else if (e.grad_upper == 0.0) {
+            r.energy_error_upper_bound = r.relative_energy_error_upper_bound = 0.0;
+            r.objective_gap_upper_bound = 0.0;
+        } else {
+            r.energy_error_upper_bound = r.relative_energy_error_upper_bound = kInf;
+            r.objective_gap_upper_bound = kInf;
+        }
+        set_outcome(r, e, reg, tol);
+    }
+    __syncthreads();
+}
+
+// The base contract and the ridge correction's preliminaries, as
+// base_contract_kernel and ridge_prelim_kernel, from the products' sums.
+__global__ void __launch_bounds__(kContractThreads)
+base_fused_kernel(ValState* vs, const VectorStats* b, Model mdl, long long m, long long n,
+                  double reg, double tol, int can_refine) {
+    __shared__ NormResult nr;
+    __shared__ Interval iv[6];
+    __shared__ double norm[6], err[4], aux[4];
+    __shared__ Envelope e;
+    __shared__ ValidationOutput r;
+    __shared__ int general;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    if (t < 6) {
+        const double mx[6] = {b->max_abs, vs->x.max_abs, vs->ax.max_t, vs->ax.max_out, vs->at.max_t,
+                              vs->at.max_out};
+        const double sq[6] = {b->sumsq, vs->x.sumsq, vs->ax.sq_t, vs->ax.sq_out, vs->at.sq_t,
+                              vs->at.sq_out};
+        set_norm(nr, t, mx[t], sq[t], t == 0 || t == 2 || t == 3 ? m : n);
+    }
+    __syncthreads();
+    if (t == 0) {
+        general = b->nonfinite || vs->x.nonfinite || vs->ax.nonfinite || vs->at.nonfinite;
+        for (int i = 0; i < 6; ++i) general |= !plain_range(nr.max_abs[i]);
+    }
+    // norms (warp 1) beside their intervals (warp 0)
+    if (warp == 1 && lane < 6) norm[lane] = euclid(nr, lane);
+    if (warp == 0 && lane < 6) iv[lane] = nint(nr, lane);
+    __syncthreads();
+    if (general) {
+        if (t == 0) {
+            vs->general = 1;
+            vs->need_refine = vs->need_correction = 0;
+        }
+        return;
+    }
+    const Interval bn = iv[0], xn = iv[1], an = iv[2], rn = iv[3], tn = iv[4], gn = iv[5];
+    const bool ok = model_ok(mdl);
+    if (lane == 0) {
+        const double u = fpb::kUnitRoundoff;
+        if (warp == 0) err[0] = callback_radius(mdl, false, xn.upper, m, u);
+        if (warp == 1) err[1] = one_op_radius(rn.upper, an.upper > 0.0 || bn.upper > 0.0, m, u);
+        if (warp == 2) err[2] = callback_radius(mdl, true, rn.upper, n, u);
+        if (warp == 3) err[3] = one_op_radius(gn.upper, reg > 0.0 && xn.upper > 0.0, n, u);
+    }
+    __syncthreads();
+    const double apply_err = err[0], t_err = err[2];
+    const Interval true_a = enlarge(an, apply_err);
+    if (lane == 0) {
+        if (warp == 0)
+            aux[0] = xn.upper > 0.0
+                         ? fpb::down_div(fpb::down_diff(an.lower, apply_err), xn.upper) : 0.0;
+        if (warp == 1)
+            aux[1] = rn.upper > 0.0 ? fpb::down_div(fpb::down_diff(tn.lower, t_err), rn.upper) : 0.0;
+        if (warp == 2) aux[2] = augmented(true_a, xn, reg).lower;
+        if (warp == 3) {
+            const double rr = sqrt(reg);
+            memset(&r, 0, sizeof(r));
+            r.residual_norm = norm[3];
+            r.normal_residual_norm = norm[5];
+            r.solution_norm = norm[1];
+            r.solution_energy_norm = hypot(norm[2], rr * norm[1]);
+            r.augmented_residual_norm = hypot(norm[3], rr * norm[1]);
+            r.augmented_operator_norm_lower_bound = rr;
+            r.objective = norm[3] * norm[3] + reg * norm[1] * norm[1];
+            r.ridge_base_energy_error_upper_bound = __builtin_nan("");
+            r.ridge_corrected_energy_error_upper_bound = __builtin_nan("");
+            r.ridge_correction_gamma = __builtin_nan("");
+            r.ridge_correction_z_h_z = __builtin_nan("");
+            r.ridge_correction_two_abs_z_t_q = __builtin_nan("");
+            r.ridge_correction_q_norm_squared = __builtin_nan("");
+            r.ridge_correction_disposition = RC_NA;
+        }
+    }
+    __syncthreads();
+    if (t == 0) {
+        memset(&e, 0, sizeof(e));
+        e.op_upper = mdl.upper;
+        e.res_upper = e.grad_upper = e.sol_upper = e.grad_radius = kInf;
+        if (ok) {
+            const double res_err = fpb::up_add(apply_err, err[1]);
+            const Interval true_res = enlarge(rn, res_err);
+            const double prop = fpb::up_mul(e.op_upper, res_err);
+            const double g_err = fpb::up_add(fpb::up_add(t_err, prop), err[3]);
+            e.res_lower = true_res.lower;
+            e.res_upper = true_res.upper;
+            e.grad_upper = enlarge(gn, g_err).upper;
+            e.sol_lower = xn.lower;
+            e.sol_upper = xn.upper;
+            e.b_lower = fmax(0.0, bn.lower);
+            e.energy_lower = aux[2];
+            e.grad_radius = g_err;
+            e.certified = isfinite(e.res_upper) && isfinite(e.grad_upper) &&
+                          isfinite(e.sol_upper) && isfinite(e.op_upper);
+            e.op_lower = fmax(fmax(mdl.lower, aux[0]), aux[1]);
+        }
+        r.operator_norm_lower_bound = e.op_lower;
+    }
+    __syncthreads();
+    certified_contract_block(r, e, reg, tol, false, 0.0);
+    if (t == 0) {
+        vs->nr = nr;
+        vs->env = e;
+        vs->bnorm = norm[0];
+        vs->general = 0;
+        vs->need_refine = can_refine && r.status != ST_SUCCESS && e.certified &&
+                          e.grad_radius >= r.normal_residual_norm;
+        vs->out = r;
+        vs->need_correction = 0;
+        if (!vs->need_refine) ridge_prelim(vs, reg);
+        vs->ran_correction_a = vs->need_correction;
+        vs->ran_correction_at = 0;
+    }
+}
+
+// d = g / ||g|| with its statistics.
+__global__ void correction_d_kernel(const double* g, ValState* vs, double* d, long long n,
+                                    double* partials, unsigned* ticket) {
+    if (!vs->need_correction) return;
+    const double s = vs->corr_gnorm;
+    double sq = 0.0;
+    unsigned long long mx = 0;
+    int bad = 0;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
+        const double v = g[i] / s;
+        d[i] = v;
+        add_stats(v, sq, mx, bad);
+    }
+    finish_stats(sq, mx, bad, partials, ticket, &vs->d);
+}
+
+// Stages 0 and 1 of correction_step_kernel, after A d and h = A^T A d + reg d
+// (with d . h).
+__global__ void __launch_bounds__(kContractThreads)
+correction_mid_kernel(ValState* vs, Model mdl, long long m, long long n, double reg) {
+    if (!vs->need_correction) return;
+    __shared__ NormResult nr;
+    __shared__ Interval iv[3];
+    __shared__ double err[4];
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    ValidationOutput& r = vs->out;
+    __shared__ int stop;
+    if (t == 0) {
+        set_norm(nr, 0, vs->d.max_abs, vs->d.sumsq, n);
+        set_norm(nr, 1, vs->ad.max_out, vs->ad.sq_out, m);
+        set_norm(nr, 2, vs->h.max_out, vs->h.sq_out, n);
+        stop = 0;
+        if (vs->d.nonfinite || vs->ad.nonfinite || vs->h.nonfinite ||
+            !plain_range(nr.max_abs[0]) || !plain_range(nr.max_abs[1]) ||
+            !plain_range(nr.max_abs[2])) {
+            stop = 1;
+            vs->general = 1;
+            vs->need_correction = 0;
+        }
+    }
+    __syncthreads();
+    if (stop) return;
+    if (t < 3) iv[t] = nint(nr, t);
+    __syncthreads();
+    if (lane == 0) {
+        const double u = fpb::kUnitRoundoff;
+        if (warp == 0) err[0] = callback_radius(mdl, false, iv[0].upper, m, u);
+        if (warp == 1) err[1] = callback_radius(mdl, true, iv[1].upper, n, u);
+        if (warp == 2)
+            err[2] = one_op_radius(iv[2].upper, reg > 0.0 && iv[0].upper > 0.0, n, u);
+        if (warp == 3) err[3] = vs->corr_gnorm / vs->h.dot;
+    }
+    __syncthreads();
+    if (t != 0) return;
+    vs->ran_correction_at = 1;
+    vs->corr_dn_upper = iv[0].upper;
+    vs->corr_adn_upper = iv[1].upper;
+    vs->corr_ad_err = err[0];
+    vs->corr_hn_upper = iv[2].upper;
+    const double prop = fpb::up_mul(vs->env.op_upper, err[0]);
+    vs->corr_herr = fpb::up_add(fpb::up_add(err[1], prop), err[2]);
+    vs->dot = vs->h.dot;
+    const double step = err[3];
+    if (!isfinite(vs->dot)) {
+        vs->need_correction = 0;
+    } else if (!(vs->dot > 0.0)) {
+        r.ridge_correction_disposition = RC_BAD_CURVATURE;
+        vs->need_correction = 0;
+    } else if (!(step > 0.0) || !isfinite(step)) {
+        vs->need_correction = 0;
+    } else {
+        vs->corr_step = step;
+    }
+}
+
+// q = g - step h; its last block takes stage 2 and the finish.
+__global__ void __launch_bounds__(kContractThreads)
+correction_end_kernel(const double* h, const double* g, ValState* vs, double* q, long long n,
+                      double reg, double tol, double* partials, unsigned* ticket) {
+    if (!vs->need_correction) return;
+    const double step = vs->corr_step;
+    double sq = 0.0;
+    unsigned long long mx = 0;
+    int bad = 0;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
+        const double v = fma(-step, h[i], g[i]);
+        q[i] = v;
+        add_stats(v, sq, mx, bad);
+    }
+    if (!finish_stats(sq, mx, bad, partials, ticket, &vs->q)) return;
+    __shared__ int improved;
+    if (threadIdx.x == 0) {
+        improved = 0;
+        if (vs->q.nonfinite || !plain_range(vs->q.max_abs)) {
+            vs->general = 1;
+        } else {
+            NormResult nr;
+            set_norm(nr, 3, vs->q.max_abs, vs->q.sumsq, n);
+            correction_bound(vs, nr, n, reg);
+            ValidationOutput& r = vs->out;
+            if (r.ridge_correction_disposition == RC_NOT_IMPROVED &&
+                isfinite(r.ridge_corrected_energy_error_upper_bound) &&
+                r.ridge_corrected_energy_error_upper_bound < r.energy_error_upper_bound) {
+                r.ridge_correction_disposition = RC_IMPROVED;
+                improved = 1;
+            }
+        }
+        vs->need_correction = 0;
+    }
+    __syncthreads();
+    if (improved)
+        certified_contract_block(vs->out, vs->env, reg, tol, true,
+                                 vs->out.ridge_corrected_energy_error_upper_bound);
+}
+
 int vgrid(long long n) {
     return (int)std::max<long long>(1, std::min<long long>(grid_cap(), (n + 255) / 256));
 }
@@ -604,6 +1010,12 @@ struct Validator::Impl {
     double* partials = nullptr;
     unsigned* counters = nullptr;
     cudaEvent_t ev[2];
+    // one-wait path: statistics of b, correction vectors, event pairs of the
+    // four products
+    VectorStats* b_stats = nullptr;
+    double *hv = nullptr, *q = nullptr;
+    cudaEvent_t pev[8] = {};
+    bool fused = true;  // until the operator turns out to have no fused product
 
     Impl(const DeviceOperator& o, const double* bb, double rg, cudaStream_t s)
         : op(o), b(bb), reg(rg), stream(s), m(o.rows()), n(o.cols()) {
@@ -622,10 +1034,22 @@ struct Validator::Impl {
         AMFLS_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned) * 16, stream));
         AMFLS_CUDA(cudaEventCreateWithFlags(&ev[0], cudaEventBlockingSync));
         AMFLS_CUDA(cudaEventCreateWithFlags(&ev[1], cudaEventBlockingSync));
+        for (cudaEvent_t& e : pev) AMFLS_CUDA(cudaEventCreate(&e));
+        if (reg > 0.0) {
+            alloc(hv, n);
+            alloc(q, n);
+        }
+        stream_alloc(&b_stats, sizeof(VectorStats), stream);
+        stats_kernel<<<vgrid(m), 256, 0, stream>>>(b, m, partials, counters + 10, b_stats);
+        AMFLS_LAUNCHED();
     }
     ~Impl() {
         cudaStreamSynchronize(stream);
-        for (double* p : {ax, r, atr, g, hi1, lo1, hi2, lo2, rn_hi, rn_lo, g2, partials}) stream_free(p, stream);
+        for (double* p : {ax, r, atr, g, hi1, lo1, hi2, lo2, rn_hi, rn_lo, g2, hv, q, partials})
+            stream_free(p, stream);
+        stream_free(b_stats, stream);
+        for (cudaEvent_t e : pev)
+            if (e) cudaEventDestroy(e);
         stream_free(vs, stream);
         stream_free(counters, stream);
         cudaEventDestroy(ev[0]);
@@ -678,28 +1102,121 @@ struct Validator::Impl {
 
     ValState read() {
         ValState h;
-        AMFLS_CUDA(cudaMemcpyAsync(&h, vs, sizeof(ValState), cudaMemcpyDeviceToHost, stream));
-        stream_wait(stream);
+        read_back(&h, vs, stream);
         return h;
     }
 
+    // One product of the one-wait path between its two events.
+    bool fused_product(int i, bool transpose, const double* x, Epilogue ep) {
+        ep.partials = partials;
+        ep.counter = counters + 8;
+        AMFLS_CUDA(cudaEventRecord(pev[2 * i], stream));
+        const bool done = op.product1(transpose, x, ep, stream);
+        AMFLS_CUDA(cudaEventRecord(pev[2 * i + 1], stream));
+        return done;
+    }
+
+    double product_seconds(int i) {
+        float ms = 0.0f;
+        AMFLS_CUDA(cudaEventElapsedTime(&ms, pev[2 * i], pev[2 * i + 1]));
+        return ms * 1e-3;
+    }
+
+    // The whole validation enqueued at once, with one wait; false when the
+    // general path has to decide (h then holds nothing).  h.need_refine asks
+    // for the refinement on top of this base.
+    bool run_fused(const double* x, double tol, ValState& h, double sec[6], int calls[6]) {
+        if (!fused) return false;
+        stats_kernel<<<vgrid(n), 256, 0, stream>>>(x, n, partials, counters + 10, &vs->x);
+        AMFLS_LAUNCHED();
+        Epilogue base;
+        base.out = r;
+        base.minus_vec = b;
+        base.red = &vs->ax;
+        if (!fused_product(0, false, x, base)) {
+            fused = false;
+            return false;
+        }
+        Epilogue grad;
+        grad.out = g;
+        grad.fma_vec = x;
+        grad.lambda = reg;
+        grad.red = &vs->at;
+        fused_product(1, true, r, grad);
+        base_fused_kernel<<<1, kContractThreads, 0, stream>>>(
+            vs, b_stats, mdl, m, n, reg, tol, op.supports_validation_refinement() ? 1 : 0);
+        AMFLS_LAUNCHED();
+        if (reg > 0.0) {
+            double *d = atr, *ad = ax;
+            correction_d_kernel<<<vgrid(n), 256, 0, stream>>>(g, vs, d, n, partials, counters + 10);
+            AMFLS_LAUNCHED();
+            Epilogue ep;
+            ep.out = ad;
+            ep.red = &vs->ad;
+            ep.guard = &vs->need_correction;
+            fused_product(2, false, d, ep);
+            Epilogue eh;
+            eh.out = hv;
+            eh.fma_vec = d;
+            eh.lambda = reg;
+            eh.dot_vec = d;
+            eh.red = &vs->h;
+            eh.guard = &vs->need_correction;
+            fused_product(3, true, ad, eh);
+            correction_mid_kernel<<<1, kContractThreads, 0, stream>>>(vs, mdl, m, n, reg);
+            AMFLS_LAUNCHED();
+            correction_end_kernel<<<vgrid(n), kContractThreads, 0, stream>>>(
+                hv, g, vs, q, n, reg, tol, partials, counters + 10);
+            AMFLS_LAUNCHED();
+        }
+        h = read();
+        if (h.general) return false;
+        calls[0] = calls[1] = 1;
+        sec[0] = product_seconds(0);
+        sec[1] = product_seconds(1);
+        if (h.ran_correction_a) {
+            calls[4] = 1;
+            sec[4] = product_seconds(2);
+        }
+        if (h.ran_correction_at) {
+            calls[5] = 1;
+            sec[5] = product_seconds(3);
+        }
+        return true;
+    }
+
+    ValidationOutput packed(const ValState& h, const double sec[6], const int calls[6]) {
+        ValidationOutput out = h.out;
+        for (int i = 0; i < 6; ++i) {
+            out.calls[i] = calls[i];
+            out.seconds[i] = sec[i];
+        }
+        return out;
+    }
+
     ValidationOutput run(const double* x, double tol) {
-        AMFLS_CUDA(cudaMemsetAsync(vs, 0, sizeof(ValState), stream));
         double sec[6] = {0, 0, 0, 0, 0, 0};
         int calls[6] = {0, 0, 0, 0, 0, 0};
-        timed_begin();
-        product(false, x, ax, r, b, nullptr);
-        sec[0] = timed_end();
-        calls[0] = 1;
-        timed_begin();
-        product(true, r, atr, g, nullptr, x);
-        sec[1] = timed_end();
-        calls[1] = 1;
-        norms(&vs->nr, {{b, m}, {x, n}, {ax, m}, {r, m}, {atr, n}, {g, n}});
-        base_contract_kernel<<<1, 32, 0, stream>>>(vs, mdl, m, n, reg, tol,
-                                                   op.supports_validation_refinement() ? 1 : 0);
-        AMFLS_LAUNCHED();
-        ValState h = read();
+        ValState h;
+        if (run_fused(x, tol, h, sec, calls)) {
+            if (!h.need_refine) return packed(h, sec, calls);
+        } else {
+            // general path: two-pass norms, a wait after every stage
+            AMFLS_CUDA(cudaMemsetAsync(vs, 0, sizeof(ValState), stream));
+            timed_begin();
+            product(false, x, ax, r, b, nullptr);
+            sec[0] = timed_end();
+            calls[0] = 1;
+            timed_begin();
+            product(true, r, atr, g, nullptr, x);
+            sec[1] = timed_end();
+            calls[1] = 1;
+            norms(&vs->nr, {{b, m}, {x, n}, {ax, m}, {r, m}, {atr, n}, {g, n}});
+            base_contract_kernel<<<1, 32, 0, stream>>>(vs, mdl, m, n, reg, tol,
+                                                       op.supports_validation_refinement() ? 1 : 0);
+            AMFLS_LAUNCHED();
+            h = read();
+        }
         const double* grad = g;
         if (h.need_refine) {
             auto alloc = [&](double*& p, long long cnt) {
@@ -743,10 +1260,6 @@ struct Validator::Impl {
                 // d = g / ||g||, A d, A^T A d + lambda d, d.h, q = g - step h
                 double* d = atr;  // reuse: the base A^T r is no longer needed
                 double* ad = ax;
-                double* hv = nullptr;
-                double* q = nullptr;
-                AMFLS_CUDA(cudaMallocAsync(&hv, sizeof(double) * n, stream));
-                AMFLS_CUDA(cudaMallocAsync(&q, sizeof(double) * n, stream));
                 scale_kernel<<<vgrid(n), 256, 0, stream>>>(grad, vs, d, n);
                 AMFLS_LAUNCHED();
                 timed_begin();
@@ -788,19 +1301,12 @@ struct Validator::Impl {
                         AMFLS_LAUNCHED();
                     }
                 }
-                AMFLS_CUDA(cudaFreeAsync(hv, stream));
-                AMFLS_CUDA(cudaFreeAsync(q, stream));
             }
         }
         finish_kernel<<<1, 32, 0, stream>>>(vs, reg, tol);
         AMFLS_LAUNCHED();
         h = read();
-        ValidationOutput out = h.out;
-        for (int i = 0; i < 6; ++i) {
-            out.calls[i] = calls[i];
-            out.seconds[i] = sec[i];
-        }
-        return out;
+        return packed(h, sec, calls);
     }
 };
 

@@ -26,6 +26,7 @@
 // (or an earlier one) stopped, so a whole run of levels up to the next
 // checkpoint is enqueued without a host round trip.
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -74,7 +75,25 @@ void stream_wait(cudaStream_t stream) {
         ev.device = dev;
     }
     AMFLS_CUDA(cudaEventRecord(ev.e, stream));
+    const auto t0 = std::chrono::steady_clock::now();
+    do {
+        const cudaError_t q = cudaEventQuery(ev.e);
+        if (q == cudaSuccess) return;
+        if (q != cudaErrorNotReady) check_cuda(q, "cudaEventQuery");
+    } while (std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(60));
     AMFLS_CUDA(cudaEventSynchronize(ev.e));
+}
+
+unsigned char* pinned_page() {
+    struct Page {
+        void* p = nullptr;
+        ~Page() {
+            if (p) cudaFreeHost(p);
+        }
+    };
+    thread_local Page page;
+    if (!page.p) AMFLS_CUDA(cudaHostAlloc(&page.p, kPinnedBytes, cudaHostAllocPortable));
+    return static_cast<unsigned char*>(page.p);
 }
 
 namespace {
@@ -1242,8 +1261,7 @@ void Workspace::initialize(const double* d_aux, int aux_cols) {
     set.count = 1;
     norm_passes(set, nr, partials_, counter_ + 1, stream_);
     NormResult h{};
-    AMFLS_CUDA(cudaMemcpyAsync(&h, nr, sizeof(NormResult), cudaMemcpyDeviceToHost, stream_));
-    stream_wait(stream_);
+    read_back(&h, nr, stream_);
     AMFLS_CUDA(cudaFreeAsync(nr, stream_));
     if (h.nonfinite[0]) throw std::invalid_argument("block Golub-Kahan right-hand side must be finite");
     b_norm_ = euclid_from(h, 0);
@@ -1498,8 +1516,7 @@ bool Workspace::advance_level() {
 }
 
 void Workspace::sync() {
-    AMFLS_CUDA(cudaMemcpyAsync(&host_, dstate_, sizeof(DevState), cudaMemcpyDeviceToHost, stream_));
-    stream_wait(stream_);
+    read_back(&host_, dstate_, stream_);
     lease_.release();
     if (host_.barrier_timeout)
         throw std::runtime_error("resident level kernel: a grid barrier timed out");
@@ -1519,6 +1536,7 @@ void Workspace::take_operator_seconds(double& a_seconds, double& at_seconds) {
 void Workspace::solve_projected(double* d_x) {
     const int k = host_.k;
     projected_flags_ = 0;
+    pending_flags_ = nullptr;
     if (k == 0) {
         AMFLS_CUDA(cudaMemsetAsync(d_x, 0, sizeof(double) * n_, stream_));
         return;
@@ -1542,10 +1560,18 @@ void Workspace::solve_projected(double* d_x) {
         V_->device_table(), n_, k, y, nullptr, d_x, 0, partials_, counter_ + 5, dstate_, kHookNone,
         m_, 0, 1);
     AMFLS_LAUNCHED();
-    double st[8];
-    AMFLS_CUDA(cudaMemcpyAsync(st, qr_state_, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream_));
-    stream_wait(stream_);
-    projected_flags_ = (int)st[5];
+    // the flags arrive with the next wait on the stream
+    pending_flags_ = reinterpret_cast<const double*>(pinned_page() + kPinnedBytes / 2);
+    AMFLS_CUDA(cudaMemcpyAsync(pinned_page() + kPinnedBytes / 2, qr_state_ + 5, sizeof(double),
+                               cudaMemcpyDeviceToHost, stream_));
+}
+
+int Workspace::projected_flags() {
+    if (pending_flags_) {
+        projected_flags_ = (int)*pending_flags_;
+        pending_flags_ = nullptr;
+    }
+    return projected_flags_;
 }
 
 namespace {

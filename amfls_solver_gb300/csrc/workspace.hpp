@@ -97,11 +97,12 @@ public:
     const StepAudit& last_step_audit() const { return host_.audit; }
     const DevState& state() const { return host_; }
 
-    // Projected solve (krylov_workspace.cpp:833-909): writes the candidate
-    // x = V y into d_x (n).  Returns false when the projected problem was
-    // flagged as numerically rank deficient (see projected_flags()).
+    // Projected solve (krylov_workspace.cpp:833-909): enqueues the candidate
+    // x = V y into d_x (n).
     void solve_projected(double* d_x);
-    int projected_flags() const { return projected_flags_; }
+    // Flags of the last projected solve (numerically rank deficient); valid
+    // once the stream has been waited for after it.
+    int projected_flags();
 
     // accumulated device timings of search operator calls since the last call
     void take_operator_seconds(double& a_seconds, double& at_seconds);
@@ -216,6 +217,7 @@ private:
     double* qr_ = nullptr;     // rho, theta, phi (3 x tcap) + y (tcap)
     double* qr_state_ = nullptr;  // [c, s, rhobar, phibar, processed]
     int projected_flags_ = 0;
+    const double* pending_flags_ = nullptr;
     // one width-one level captured as the body of a device-side WHILE loop
     cudaStream_t capture_stream_ = nullptr;
     cudaGraph_t graph_ = nullptr;
