@@ -215,7 +215,7 @@ private:
     int tcap_ = 0;
     // incremental Givens QR of [T; sqrt(lambda) I]
     double* qr_ = nullptr;     // rho, theta, phi (3 x tcap) + y (tcap)
-    double* qr_state_ = nullptr;  // [c, s, rhobar, phibar, processed]
+    double* qr_state_ = nullptr;  // state of projected_solve_kernel
     int projected_flags_ = 0;
     const double* pending_flags_ = nullptr;
     // one width-one level captured as the body of a device-side WHILE loop
