@@ -5,19 +5,20 @@
 // A pool of host worker threads, each with its own non-blocking CUDA
 // stream, takes problems from a shared queue ordered by estimated cost
 // (largest first, the LPT rule, so the last problems to start are the
-// short ones).  Every solve runs on its worker's stream, so the GPU
-// interleaves the levels of up to `workers` problems; small problems, whose
-// levels are launch- and latency-bound, share the SMs instead of leaving
-// them idle.  A single solve runs each
-// checkpoint interval as one CUDA graph (a conditional WHILE node over the
-// level), but graphs launched on different streams were measured to run one
-// at a time (48 problems, 16 workers: 12.5 s with those graphs, 10.5-12.3 s
-// with plain graphs of 2-32 levels, 7.9 s with the level kernels launched
-// from the host), so a batch with more than one worker launches from the
-// host.
+// short ones).  The levels of a CSR problem run in the resident level kernel on
+// a share of the SMs (sm_shares below), so that up to `workers` problems
+// really run side by side: a small problem's level is a chain of latencies
+// that leaves most of a whole GPU idle, and its work takes no longer on ten
+// SMs than it waits anyway.  Sixteen CSR problems of up to 20000 x 4000, 16
+// workers: 337 ms with the level kernels launched from the host, 261 ms with
+// the waits of the validation taken out, 128 ms with the shares.  Other operators'
+// levels are launched from the host when there is more than one worker
+// (graphs of different streams ran one at a time: 48 problems, 16 workers,
+// 12.5 s against 7.9 s).
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <exception>
 #include <numeric>
 #include <stdexcept>
@@ -28,15 +29,57 @@
 #include "batch.hpp"
 #include "common.cuh"
 #include "csr_operator.hpp"
+#include "resident_levels.hpp"
 
 namespace amfls_gpu {
 
 namespace {
 
+constexpr int kMinShare = 4;
+// Streams of resident solves that run side by side: the driver maps streams to
+// eight hardware queues (its default), and kernels behind a resident one in
+// the same queue wait for it.  1500-column problems on 8 SMs each: 8 in 50 ms, 9
+// in 75 ms, 16 in 171 ms; two rounds of eight on 17 SMs take 68 ms.
+constexpr int kResidentStreams = 8;
+
+// Work of a problem's level, in FP64 operations of the resident kernel: the
+// sweeps of a basis that grows with the columns (n k each, k about an eighth
+// of n on average) and the products (a gather costs about two operations).
 double cost_estimate(const DeviceOperator& op) {
+    ResidentOperator view;
+    const double n = op.cols();
+    if (op.resident(&view)) return 0.25 * n * n + 4.0 * (double)view.nonzeros;
     if (const auto* csr = dynamic_cast<const CsrOperator*>(&op))
-        return (double)csr->nonzeros() + op.rows() + op.cols();
-    return (double)op.rows() * op.cols();
+        return 0.25 * n * n + 4.0 * (double)csr->nonzeros();
+    return 4.0 * op.rows() * n;
+}
+
+// SMs of each problem in LPT order, from the batch alone (so that a repeat
+// gives the same sums): of the `workers` problems that run from position p
+// on, each takes the part of the SMs that the square root of its work is of
+// theirs (which makes the sum of work / SMs smallest; in proportion to the
+// work the 16 problems take as long with 8 in flight, 128 ms, and 147 instead
+// of 129 ms with 4).  A tenth of the SMs stays free for the checkpoints'
+// kernels, which find no room beside a resident block.
+std::vector<int> sm_shares(const std::vector<BatchItem>& items, const std::vector<int>& order,
+                           int workers) {
+    const int count = (int)order.size(), sms = sm_count();
+    std::vector<double> weight(count, 0.0);
+    for (int p = 0; p < count; ++p) {
+        ResidentOperator view;
+        const DeviceOperator& op = *items[order[p]].op;
+        if (op.resident(&view)) weight[p] = std::sqrt(cost_estimate(op));
+    }
+    std::vector<int> share(count, 0);
+    for (int p = 0; p < count; ++p) {
+        // the last `workers` problems run beside each other to the end
+        const int first = std::max(0, std::min(p, count - workers));
+        double sum = 0.0;
+        for (int q = first; q < std::min(count, first + workers); ++q) sum += weight[q];
+        if (weight[p] > 0.0)
+            share[p] = std::clamp((int)(0.9 * sms * weight[p] / sum), kMinShare, sms);
+    }
+    return share;
 }
 
 }  // namespace
@@ -62,6 +105,11 @@ std::vector<BatchOutcome> solve_amfls_batch(const std::vector<BatchItem>& items,
             throw std::invalid_argument("each problem of a batch needs its own operator");
     }
     workers = std::min(workers, count);
+    const bool resident = std::all_of(items.begin(), items.end(), [](const BatchItem& it) {
+        ResidentOperator view;
+        return it.op->resident(&view);
+    });
+    if (resident) workers = std::min(workers, kResidentStreams);
     std::vector<int> order(count);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
@@ -69,6 +117,7 @@ std::vector<BatchOutcome> solve_amfls_batch(const std::vector<BatchItem>& items,
     });
     int device = 0;
     AMFLS_CUDA(cudaGetDevice(&device));
+    const std::vector<int> share = sm_shares(items, order, workers);
     std::atomic<int> next{0};
     const auto t0 = std::chrono::steady_clock::now();
     auto work = [&](int w) {
@@ -87,10 +136,10 @@ std::vector<BatchOutcome> solve_amfls_batch(const std::vector<BatchItem>& items,
             const auto ts = std::chrono::steady_clock::now();
             try {
                 SolveOptions opts = items[i].options;
-                // CUDA graphs of different streams were measured to run
-                // their work one graph at a time: concurrent solves launch
-                // their level kernels from the host instead
-                if (workers > 1) opts.use_graphs = false;
+                if (workers > 1) {
+                    opts.use_graphs = false;
+                    opts.resident_sms = share[k];
+                }
                 o.result = solve_amfls(*items[i].op, items[i].b, opts, items[i].x, s);
                 o.ok = true;
             } catch (const std::exception& e) {

@@ -65,8 +65,7 @@ void grow(T*& p, long long& cap, long long need, long long keep, cudaStream_t s)
 }  // namespace
 
 void Workspace::push_state() {
-    AMFLS_CUDA(cudaMemcpyAsync(dstate_, &host_, sizeof(DevState), cudaMemcpyHostToDevice, stream_));
-    stream_wait(stream_);
+    put(dstate_, host_, stream_);
 }
 
 void Workspace::upload(double* dst, const std::vector<double>& src) {

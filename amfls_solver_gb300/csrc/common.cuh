@@ -55,29 +55,88 @@ inline void stream_free(const void* p, cudaStream_t s) {
 // buffers.  Called by each solve; takes effect once per device.
 void keep_pool_memory();
 
-// Waits until the work enqueued on `stream` so far has finished: polls for a
-// few tens of microseconds (short waits then end without a thread wake-up),
-// then blocks the calling thread on a blocking-sync event (concurrent solves
-// on many host threads leave the CPU cores to the threads that launch work).
+// Small exchanges between a solve and its host thread.
+//
+// Copies of a few hundred bytes go through kernels, not through the copy
+// engines: a device-to-host copy queued behind a long resident kernel holds
+// its engine's queue, and with it the copies of every other solve that shares
+// the queue.  Results land in pinned host memory that the GPU writes, followed
+// by a sequence number the host polls, so that a wait costs neither a thread
+// wake-up nor a driver call.
+
+// Pinned host memory of the calling thread, freed with the thread: the
+// landing place of small reads.  The first half belongs to reads that are
+// waited for at once, the second half to values read after the next wait.
+constexpr size_t kPinnedBytes = 1 << 16;
+struct HostPage {
+    unsigned char* data = nullptr;
+    unsigned* flag = nullptr;  // last sequence number the GPU has reached
+    unsigned seq = 0;
+};
+HostPage& host_page();
+
+// Waits until the page's flag has reached seq: polls, then yields the core
+// between polls, then sleeps between them (many solves on many host threads);
+// a failed kernel ends the wait with its error.
+void wait_flag(const HostPage& page, unsigned seq, cudaStream_t stream);
+
+// Waits until the work enqueued on `stream` so far has finished.
 void stream_wait(cudaStream_t stream);
 
-// A page of pinned host memory of the calling thread, freed with the thread:
-// the landing place of the small device-to-host reads of a solve.  The first
-// half belongs to state that is read and used at once, the second half to
-// the projected solve's flags (read after the next wait).
-constexpr size_t kPinnedBytes = 8192;
-unsigned char* pinned_page();
+#if defined(__CUDACC__)
+static __global__ void copy_out_kernel(const unsigned* src, unsigned* dst, int words,
+                                       unsigned* flag, unsigned seq) {
+    for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+    __threadfence_system();
+    __syncthreads();
+    if (flag && threadIdx.x == 0) *(volatile unsigned*)flag = seq;
+}
+
+// *dst = value, in stream order (values up to the size of a kernel argument).
+template <typename T>
+__global__ void put_kernel(T* dst, T value) {
+    const unsigned* src = reinterpret_cast<const unsigned*>(&value);
+    unsigned* out = reinterpret_cast<unsigned*>(dst);
+    for (int i = threadIdx.x; i < (int)(sizeof(T) / sizeof(unsigned)); i += blockDim.x)
+        out[i] = src[i];
+}
+template <typename T>
+inline void put(T* dst, const T& value, cudaStream_t stream) {
+    static_assert(sizeof(T) % sizeof(unsigned) == 0 && sizeof(T) <= 3072);
+    put_kernel<T><<<1, 64, 0, stream>>>(dst, value);
+    check_cuda(cudaGetLastError(), "kernel launch");
+    ++launch_count();
+}
+
+// Device bytes (a multiple of 4, 4-byte aligned) into the page at `offset`;
+// with `signal` the flag follows.
+inline void copy_out(const void* device, size_t bytes, size_t offset, bool signal,
+                     cudaStream_t stream) {
+    HostPage& page = host_page();
+    const int words = (int)(bytes / 4);
+    copy_out_kernel<<<1, words > 128 ? 512 : 64, 0, stream>>>(
+        static_cast<const unsigned*>(device), reinterpret_cast<unsigned*>(page.data + offset),
+        words, signal ? page.flag : nullptr, signal ? ++page.seq : 0u);
+    check_cuda(cudaGetLastError(), "kernel launch");
+    ++launch_count();
+}
 
 // Copies a small device object to the host and waits for it.
 template <typename T>
-inline void read_back(T* host, const T* device, cudaStream_t stream) {
-    static_assert(sizeof(T) <= kPinnedBytes / 2);
-    unsigned char* page = pinned_page();
-    check_cuda(cudaMemcpyAsync(page, device, sizeof(T), cudaMemcpyDeviceToHost, stream),
-               "cudaMemcpyAsync");
-    stream_wait(stream);
-    std::memcpy(host, page, sizeof(T));
+inline void read_back(T* host, const T* device, cudaStream_t stream, size_t count = 1) {
+    const size_t bytes = sizeof(T) * count;
+    if (bytes > kPinnedBytes / 2 || bytes % 4 != 0) {
+        check_cuda(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, stream),
+                   "cudaMemcpyAsync");
+        stream_wait(stream);
+        return;
+    }
+    copy_out(device, bytes, 0, true, stream);
+    const HostPage& page = host_page();
+    wait_flag(page, page.seq, stream);
+    std::memcpy(host, page.data, bytes);
 }
+#endif
 
 // Streaming multiprocessors of the current device
 // (cudaDevAttrMultiProcessorCount), queried once per device.

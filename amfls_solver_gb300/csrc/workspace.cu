@@ -26,12 +26,14 @@
 // (or an earlier one) stopped, so a whole run of levels up to the next
 // checkpoint is enqueued without a host round trip.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <stdexcept>
+#include <thread>
 #include <vector>
 
 #include <cuda_fp16.h>
@@ -57,43 +59,54 @@ void keep_pool_memory() {
     done[dev] = true;
 }
 
-void stream_wait(cudaStream_t stream) {
-    struct Event {
-        cudaEvent_t e = nullptr;
-        int device = -1;
-        ~Event() {
-            if (e) cudaEventDestroy(e);
+HostPage& host_page() {
+    struct Owner {
+        HostPage page;
+        ~Owner() {
+            if (page.data) cudaFreeHost(page.data);
         }
     };
-    thread_local Event ev;
-    int dev = 0;
-    AMFLS_CUDA(cudaGetDevice(&dev));
-    if (!ev.e || ev.device != dev) {
-        if (ev.e) cudaEventDestroy(ev.e);
-        ev.e = nullptr;
-        AMFLS_CUDA(cudaEventCreateWithFlags(&ev.e, cudaEventBlockingSync | cudaEventDisableTiming));
-        ev.device = dev;
+    thread_local Owner owner;
+    HostPage& page = owner.page;
+    if (!page.data) {
+        void* p = nullptr;
+        AMFLS_CUDA(cudaHostAlloc(&p, kPinnedBytes + 64, cudaHostAllocPortable));
+        page.data = static_cast<unsigned char*>(p);
+        page.flag = reinterpret_cast<unsigned*>(page.data + kPinnedBytes);
+        *page.flag = 0;
+        page.seq = 0;
     }
-    AMFLS_CUDA(cudaEventRecord(ev.e, stream));
-    const auto t0 = std::chrono::steady_clock::now();
-    do {
-        const cudaError_t q = cudaEventQuery(ev.e);
-        if (q == cudaSuccess) return;
-        if (q != cudaErrorNotReady) check_cuda(q, "cudaEventQuery");
-    } while (std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(60));
-    AMFLS_CUDA(cudaEventSynchronize(ev.e));
+    return page;
 }
 
-unsigned char* pinned_page() {
-    struct Page {
-        void* p = nullptr;
-        ~Page() {
-            if (p) cudaFreeHost(p);
+void wait_flag(const HostPage& page, unsigned seq, cudaStream_t stream) {
+    const volatile unsigned* flag = page.flag;
+    const auto reached = [&] { return (int)(*flag - seq) >= 0; };
+    const auto t0 = std::chrono::steady_clock::now();
+    auto checked = t0;
+    while (!reached()) {
+        const auto now = std::chrono::steady_clock::now();
+        if (now - checked > std::chrono::milliseconds(2)) {
+            // done without the flag: the kernel failed, or its last write is
+            // on its way
+            const cudaError_t e = cudaStreamQuery(stream);
+            if (e != cudaSuccess && e != cudaErrorNotReady) check_cuda(e, "cudaStreamQuery");
+            if (e == cudaSuccess && !reached()) AMFLS_CUDA(cudaStreamSynchronize(stream));
+            checked = now;
         }
-    };
-    thread_local Page page;
-    if (!page.p) AMFLS_CUDA(cudaHostAlloc(&page.p, kPinnedBytes, cudaHostAllocPortable));
-    return static_cast<unsigned char*>(page.p);
+        if (now - t0 > std::chrono::milliseconds(20))
+            std::this_thread::sleep_for(std::chrono::microseconds(20));
+        else if (now - t0 > std::chrono::microseconds(100))
+            std::this_thread::yield();
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+}
+
+void stream_wait(cudaStream_t stream) {
+    HostPage& page = host_page();
+    copy_out_kernel<<<1, 32, 0, stream>>>(nullptr, nullptr, 0, page.flag, ++page.seq);
+    AMFLS_CUDA(cudaGetLastError());
+    wait_flag(page, page.seq, stream);
 }
 
 namespace {
@@ -1183,6 +1196,17 @@ projected_solve_kernel(const double* alpha, const double* beta, const double* g,
 
 // ------------------------------------------------------------ panels ----
 
+namespace {
+template <typename T>
+struct PointerChunk {
+    T* p[64];
+};
+template <typename T>
+__global__ void put_pointers_kernel(T** table, PointerChunk<T> c, int count) {
+    if ((int)threadIdx.x < count) table[threadIdx.x] = c.p[threadIdx.x];
+}
+}  // namespace
+
 template <typename T>
 PanelStoreT<T>::PanelStoreT(int n, int max_panels, cudaStream_t stream)
     : n_(n), stream_(stream), table_cap_(std::max(1, max_panels)) {
@@ -1212,10 +1236,13 @@ void PanelStoreT<T>::ensure_columns(int cols) {
         AMFLS_CUDA(cudaMemsetAsync(p, 0, sizeof(T) * 32 * static_cast<size_t>(n_), stream_));
         host_.push_back(p);
     }
-    // host_ never reallocates (reserved to table_cap_), so the async copy
-    // reads stable memory
-    AMFLS_CUDA(cudaMemcpyAsync(table_ + first, host_.data() + first,
-                               sizeof(T*) * (need - first), cudaMemcpyHostToDevice, stream_));
+    for (int i = first; i < need; i += 64) {
+        PointerChunk<T> c{};
+        const int count = std::min(64, need - i);
+        std::copy_n(host_.data() + i, count, c.p);
+        put_pointers_kernel<<<1, 64, 0, stream_>>>(table_ + i, c, count);
+        AMFLS_LAUNCHED();
+    }
 }
 
 template class PanelStoreT<double>;
@@ -1297,13 +1324,10 @@ Workspace::Workspace(const DeviceOperator& op, const double* d_b, double regular
                          stream_);
             stream_alloc(&resident_barrier_, sizeof(unsigned), stream_);
         }
-        AMFLS_CUDA(cudaStreamCreateWithFlags(&capture_stream_, cudaStreamNonBlocking));
         std::memset(&host_, 0, sizeof(host_));
         host_.reliable = 1;
         host_.basis_limit = basis_limit_;
-        AMFLS_CUDA(cudaMemcpyAsync(dstate_, &host_, sizeof(DevState), cudaMemcpyHostToDevice,
-                                   stream_));
-        stream_wait(stream_);
+        put(dstate_, host_, stream_);
     } catch (...) {  // e.g. out of device memory part way: free what was allocated
         release();
         throw;
@@ -1441,14 +1465,13 @@ void Workspace::initialize(const double* d_aux, int aux_cols) {
         scale_copy_kernel<<<std::max<long long>(1, std::min<long long>(grid_cap(), (m_ + 255) / 256)), 256, 0,
                             stream_>>>(b_, U_, m_, inv);
         AMFLS_LAUNCHED();
-        AMFLS_CUDA(cudaMemcpyAsync(g_, &b_norm_, sizeof(double), cudaMemcpyHostToDevice, stream_));
+        put(g_, b_norm_, stream_);
         host_.left_width = 1;
         host_.rows_t = 1;
         host_.active_first = 0;
     }
     std::memset(&host_.audit, 0, sizeof(host_.audit));
-    AMFLS_CUDA(cudaMemcpyAsync(dstate_, &host_, sizeof(DevState), cudaMemcpyHostToDevice, stream_));
-    stream_wait(stream_);
+    put(dstate_, host_, stream_);
     if (b_norm_ > 0.0 && aux_cols > 0) append_left_seed(d_aux, aux_cols);
 }
 
@@ -1574,6 +1597,8 @@ void Workspace::enqueue_level_kernels(cudaStream_t s, int pcap) {
 
 void Workspace::build_graph(int pcap) {
     invalidate_graph();
+    if (!capture_stream_)
+        AMFLS_CUDA(cudaStreamCreateWithFlags(&capture_stream_, cudaStreamNonBlocking));
     AMFLS_CUDA(cudaGraphCreate(&graph_, 0));
     cudaGraphConditionalHandle handle;
     AMFLS_CUDA(cudaGraphConditionalHandleCreate(&handle, graph_, 1, cudaGraphCondAssignDefault));
@@ -1731,9 +1756,8 @@ void Workspace::solve_projected(double* d_x) {
         m_, 0, 1);
     AMFLS_LAUNCHED();
     // the flags arrive with the next wait on the stream
-    pending_flags_ = reinterpret_cast<const double*>(pinned_page() + kPinnedBytes / 2);
-    AMFLS_CUDA(cudaMemcpyAsync(pinned_page() + kPinnedBytes / 2, qr_state_ + 5, sizeof(double),
-                               cudaMemcpyDeviceToHost, stream_));
+    copy_out(qr_state_ + 5, sizeof(double), kPinnedBytes / 2, false, stream_);
+    pending_flags_ = reinterpret_cast<const double*>(host_page().data + kPinnedBytes / 2);
 }
 
 int Workspace::projected_flags() {
