@@ -232,23 +232,30 @@ def counterfactual_dataset(problems, *, max_sites: int = 8) -> Dataset:
 
     from .binding import solve_amfls_replay
 
+    # The heuristic's gate weighs measured block costs, so the choices after a
+    # site, and with them a solve's time, can differ between runs (up to 40%
+    # on the dense study family): a solve counts with the fastest of a few runs.
+    def fastest(solve, runs=3):
+        best, kept = float("inf"), None
+        for _ in range(runs):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            out = solve()
+            torch.cuda.synchronize()
+            t = time.perf_counter() - t0
+            if t < best:
+                best, kept = t, out
+        return best, kept
+
     xs, ys = [], []
     for matrix, b, options in problems:
         op = matrix if isinstance(matrix, DeviceOperator) else DeviceOperator(matrix)
         solve_controlled(op, b, **options)  # warm-up
-        torch.cuda.synchronize()
-        t0 = time.perf_counter()
-        _, log = solve_controlled(op, b, **options)
-        torch.cuda.synchronize()
-        t_h = time.perf_counter() - t0
+        t_h, (_, log) = fastest(lambda: solve_controlled(op, b, **options))
         bits = [int(v) for v in log[:, 11]] if len(log) else []
         for i in range(min(len(bits), max_sites)):
             replay = bits[:i] + [1 - bits[i]]
-            torch.cuda.synchronize()
-            t0 = time.perf_counter()
-            solve_amfls_replay(op, b, replay, **options)
-            torch.cuda.synchronize()
-            t_f = time.perf_counter() - t0
+            t_f, _ = fastest(lambda: solve_amfls_replay(op, b, replay, **options))
             f = log[i, :F]
             xs.append(np.concatenate([f, [bits[i]]]))
             ys.append(0.0)
