@@ -20,6 +20,7 @@
 
 #include "block.hpp"
 #include "common.cuh"
+#include "narrow_block.hpp"
 #include "workspace.hpp"
 
 namespace amfls_gpu {
@@ -178,7 +179,8 @@ void Workspace::enter_block_mode() {
 
 Workspace::Factor Workspace::orthogonalize_and_factor(double* B, int cols, const Basis& basis,
                                                       int max_rank, double scale, int tracked,
-                                                      bool retain, double* q_out) {
+                                                      bool retain, double* q_out,
+                                                      const Projected* projected) {
     const long long rows = basis.panels ? n_ : m_;
     const int kb = basis.cols;
     Factor F;
@@ -187,7 +189,14 @@ Workspace::Factor Workspace::orthogonalize_and_factor(double* B, int cols, const
     bool coeff_finite = true;
     int passes = 0;
     double* C[2] = {nullptr, nullptr};
-    if (kb > 0 && cols > 0) {
+    if (projected) {
+        if (retain) F.coefficients = projected->coefficients;
+        coeff_finite = projected->finite;
+        for (double v : F.coefficients)
+            if (!std::isfinite(v)) coeff_finite = false;
+        resid = device_norm(B, rows * cols);
+    }
+    if (!projected && kb > 0 && cols > 0) {
         grow(coefs_, coefs_cap_, 2LL * kb * cols, 0, stream_);
         C[0] = coefs_;
         C[1] = coefs_ + (long long)kb * cols;
@@ -206,7 +215,9 @@ Workspace::Factor Workspace::orthogonalize_and_factor(double* B, int cols, const
         }
         ++passes;
     };
-    if (cols == 1 && kb > 0) {
+    if (projected) {
+        // the passes ran in the level's device chain
+    } else if (cols == 1 && kb > 0) {
         // scalar DGKS (krylov_workspace.cpp:110-170)
         const double before = device_norm(B, rows);
         project(C[0]);
@@ -381,6 +392,101 @@ int Workspace::append_left_seed(const double* d_seed, int cols) {
     return F.rank;
 }
 
+// Enqueues the level of a block of cw columns (2 .. kNarrowMax, nothing
+// capped) as device work and reads what it left behind; false when the level
+// is not of that kind and nothing was done.
+bool Workspace::narrow_level(int cw, int aw, int max_right, int old_left,
+                             narrow::LevelResult* out) {
+    const int pw = host_.prev_right_width, k = host_.k;
+    if (!narrow_levels_ || cw < 2 || cw > narrow::kNarrowMax || aw > narrow::kNarrowMax ||
+        pw > narrow::kNarrowMax || max_right != cw || cw > n_ || !op_.graph_safe() ||
+        std::min(m_ - old_left, basis_limit_ + 1 - old_left) < cw)
+        return false;
+    const bool couple = pw > 0 && aw > 0;
+    if (couple && coupling_.size() != (size_t)aw * pw)
+        throw std::logic_error("block Golub-Kahan frontier coupling dimensions are invalid");
+    V_->ensure_columns(k + cw);
+    const int P = (k + 31) / 32;
+    grow(coefs_, coefs_cap_,
+         std::max<long long>(narrow::kSquare, narrow::panel_coefficient_doubles(std::max(k, 1), cw)),
+         0, stream_);
+    grow(small_, small_cap_, 3LL * 32 * narrow::kNarrowMax, 0, stream_);
+    grow(bpart_, bpart_cap_,
+         std::max<long long>(narrow::panel_tn_partial_doubles(n_, std::max(k, 1), cw),
+                             256LL * narrow::kSquare),
+         0, stream_);
+    if (!level_) stream_alloc(&level_, sizeof(narrow::LevelResult), stream_);
+    for (cudaEvent_t& e : nev_)
+        if (!e) AMFLS_CUDA(cudaEventCreate(&e));
+    AMFLS_CUDA(cudaMemsetAsync(level_, 0, sizeof(narrow::LevelResult), stream_));
+    narrow::Factorisation &right = level_->right, &left = level_->left;
+    unsigned *norm_ticket = counter_ + 6, *gram_ticket = counter_ + 7, *panel_tickets = counter_ + 64;
+    double* const* V = V_->device_table();
+    const double unit_right = rank_revealing_cutoff(1.0, m_, n_, k, cw);
+    const double unit_left = rank_revealing_cutoff(1.0, m_, n_, aw, cw);
+    auto factorise = [&](const double* B, long long rows, narrow::Factorisation* f, double unit,
+                         double* q) {
+        narrow::cholesky_pass(B, rows, cw, 1, unit, f, bpart_, gram_ticket, stream_);
+        narrow::apply(B, f->inverse, false, cw, rows, cw, cw, BT_, 1.0, 0.0, stream_);
+        narrow::cholesky_pass(BT_, rows, cw, 2, unit, f, bpart_, gram_ticket, stream_);
+        narrow::apply(BT_, f->inverse, false, cw, rows, cw, cw, q, 1.0, 0.0, stream_);
+    };
+
+    AMFLS_CUDA(cudaEventRecord(nev_[0], stream_));
+    op_.apply_transpose(U_, cw, BR_, stream_);
+    AMFLS_CUDA(cudaEventRecord(nev_[1], stream_));
+    narrow::frobenius2(BR_, (long long)n_ * cw, &right.scale2, bpart_, norm_ticket, stream_);
+    if (couple) {
+        narrow::Small m{};
+        std::copy(coupling_.begin(), coupling_.end(), m.v);
+        const int first = host_.prev_right_first;
+        narrow::spread_coefficients(m, first, pw, aw, small_, stream_);
+        narrow::panel_nn(V, n_, first / 32, (first + pw + 31) / 32, small_, aw, BR_, stream_);
+    }
+    for (int pass = 0; pass < 2 && k > 0; ++pass) {  // block CGS2
+        narrow::panel_tn(V, n_, k, BR_, cw, coefs_, bpart_, panel_tickets, &right.nonfinite,
+                         stream_);
+        narrow::panel_nn(V, n_, 0, P, coefs_, cw, BR_, stream_);
+    }
+    factorise(BR_, n_, &right, unit_right, BQ_);
+
+    AMFLS_CUDA(cudaEventRecord(nev_[2], stream_));
+    op_.apply(BQ_, cw, BL_, stream_);
+    AMFLS_CUDA(cudaEventRecord(nev_[3], stream_));
+    narrow::frobenius2(BL_, (long long)m_ * cw, &left.scale2, bpart_, norm_ticket, stream_);
+    if (aw > 0)
+        narrow::apply(U_, right.factor, true, cw, m_, aw, cw, BL_, -1.0, 1.0, stream_);
+    for (int pass = 0; pass < 2 && aw > 0; ++pass) {
+        narrow::gram(U_, BL_, m_, aw, cw, coefs_, level_->coefficients, bpart_, gram_ticket,
+                     &left.nonfinite, stream_);
+        narrow::apply(U_, coefs_, false, aw, m_, aw, cw, BL_, -1.0, 1.0, stream_);
+    }
+    factorise(BL_, m_, &left, unit_left, U2_);
+    narrow::gram(U2_, b_, m_, cw, 1, level_->g, nullptr, bpart_, gram_ticket, nullptr, stream_);
+    narrow::append(V, n_, k, BQ_, cw, level_, stream_);
+    read_back(out, level_, stream_);
+    // squares that left FP64's range: the general path starts the level anew
+    auto plain = [](double v) { return v > 1e-250 && v < 1e250; };
+    return out->right.ok
+               ? out->left.ok || plain(out->left.scale2)
+               : plain(out->right.scale2);
+}
+
+double Workspace::narrow_seconds(int half) {
+    float ms = 0.0f;
+    AMFLS_CUDA(cudaEventElapsedTime(&ms, nev_[2 * half], nev_[2 * half + 1]));
+    return static_cast<double>(ms) * 1e-3;
+}
+
+Workspace::Factor Workspace::narrow_factor(const narrow::Factorisation& f, int cols,
+                                           int basis_cols) {
+    Factor F;
+    F.rank = cols;
+    F.cutoff = rank_revealing_cutoff(std::sqrt(f.scale2), m_, n_, basis_cols, cols);
+    F.factor.assign(f.factor, f.factor + (size_t)cols * cols);
+    return F;
+}
+
 bool Workspace::block_level() {
     StepAudit a;
     std::memset(&a, 0, sizeof(a));
@@ -402,16 +508,25 @@ bool Workspace::block_level() {
     ensure_block_capacity(cw);
     ensure_u_capacity(cw);
 
+    const int max_right = std::min(cw, basis_limit_ - host_.k);
+    // the whole level as device work first, when its width allows; `level`
+    // then holds its factorisations (see narrow_block.hpp)
+    narrow::LevelResult level{};
+    const bool narrow = narrow_level(cw, aw, max_right, old_left, &level);
+    const bool right_done = narrow && level.right.ok;
+    const bool left_done = right_done && level.left.ok;
+
     // right half-step: A^T [U P] - V_prev coupling^T, projected off V
-    const double t_at = timed_apply(true, U_, cw, BR_);
+    const double t_at = narrow ? narrow_seconds(0) : timed_apply(true, U_, cw, BR_);
     host_.at_ns += static_cast<unsigned long long>(t_at * 1e9);
     host_.search_at_calls += 1;
     host_.search_at_columns += cw;
     host_.pending = 0;
     pending_requested_ = 0;
     pending_retained_ = 0;
-    const double right_scale = device_norm(BR_, (long long)n_ * cw);
-    if (host_.prev_right_width > 0 && aw > 0) {
+    const double right_scale =
+        narrow ? std::sqrt(level.right.scale2) : device_norm(BR_, (long long)n_ * cw);
+    if (!narrow && host_.prev_right_width > 0 && aw > 0) {
         const int pw = host_.prev_right_width;
         if (coupling_.size() != (size_t)aw * pw)
             throw std::logic_error("block Golub-Kahan frontier coupling dimensions are invalid");
@@ -422,10 +537,15 @@ bool Workspace::block_level() {
         panel_nn(V_->device_table(), n_, host_.prev_right_first, pw, small_, aw, BR_, n_, -1.0,
                  stream_);
     }
-    const int max_right = std::min(cw, basis_limit_ - host_.k);
     V_->ensure_columns(host_.k + std::max(1, max_right));
-    const Factor F = orthogonalize_and_factor(BR_, cw, Basis{true, nullptr, host_.k}, max_right,
-                                              right_scale, aw, false, BQ_);
+    Factor F;
+    if (right_done) {
+        F = narrow_factor(level.right, cw, host_.k);
+    } else {
+        const Projected off{level.right.nonfinite == 0, {}};
+        F = orthogonalize_and_factor(BR_, cw, Basis{true, nullptr, host_.k}, max_right, right_scale,
+                                     aw, false, BQ_, narrow ? &off : nullptr);
+    }
     StepAudit& au = host_.audit;
     au.retained_right_width = F.rank;
     au.right_rank_cutoff = F.cutoff;
@@ -448,12 +568,13 @@ bool Workspace::block_level() {
     }
 
     // left half-step: A q - U Fa^T, projected off U
-    const double t_a = timed_apply(false, BQ_, r, BL_);
+    const double t_a = right_done ? narrow_seconds(1) : timed_apply(false, BQ_, r, BL_);
     host_.a_ns += static_cast<unsigned long long>(t_a * 1e9);
     host_.search_a_calls += 1;
     host_.search_a_columns += r;
-    const double left_scale = device_norm(BL_, (long long)m_ * r);
-    if (aw > 0) {
+    const double left_scale =
+        right_done ? std::sqrt(level.left.scale2) : device_norm(BL_, (long long)m_ * r);
+    if (!right_done && aw > 0) {
         std::vector<double> ct((size_t)aw * r);  // Fa^T, Fa = factor[:, :aw]
         for (int i = 0; i < aw; ++i)
             for (int c = 0; c < r; ++c) ct[i + (size_t)c * aw] = F.factor[c + (size_t)i * r];
@@ -461,8 +582,17 @@ bool Workspace::block_level() {
         ts_nn(U_, m_, small_, m_, aw, r, BL_, m_, -1.0, 1.0, stream_);
     }
     const int max_left = std::min({r, m_ - old_left, basis_limit_ + 1 - old_left});
-    const Factor FL = orthogonalize_and_factor(BL_, r, Basis{false, U_, aw}, max_left, left_scale, 0,
-                                               true, U2_);
+    Factor FL;
+    if (left_done) {
+        FL = narrow_factor(level.left, r, aw);
+        FL.coefficients.assign(level.coefficients, level.coefficients + (size_t)aw * r);
+    } else {
+        Projected off{level.left.nonfinite == 0, {}};
+        if (right_done)
+            off.coefficients.assign(level.coefficients, level.coefficients + (size_t)aw * r);
+        FL = orthogonalize_and_factor(BL_, r, Basis{false, U_, aw}, max_left, left_scale, 0, true,
+                                      U2_, right_done ? &off : nullptr);
+    }
     au.retained_next_left_width = FL.rank;
     au.left_rank_cutoff = FL.cutoff;
     au.left_discarded_residual_norm = FL.discarded;
@@ -476,12 +606,14 @@ bool Workspace::block_level() {
         return false;
     }
     const int nlw = FL.rank;
-    panel_append(V_->device_table(), n_, host_.k, BQ_, r, stream_);
+    if (!left_done) panel_append(V_->device_table(), n_, host_.k, BQ_, r, stream_);
     host_.k += r;
 
     // level record: G = Fa^T + left coefficients, N = left factor, g = q^T b
     std::vector<double> gnew(nlw);
-    if (nlw > 0) {
+    if (left_done) {
+        std::copy_n(level.g, nlw, gnew.begin());
+    } else if (nlw > 0) {
         grow(bpart_, bpart_cap_, ts_tn_partial_doubles(m_, nlw, 1), 0, stream_);
         ts_tn(U2_, m_, b_, m_, m_, nlw, 1, small_, bpart_, nullptr, stream_);
         AMFLS_CUDA(cudaMemcpyAsync(gnew.data(), small_, sizeof(double) * nlw, cudaMemcpyDeviceToHost,

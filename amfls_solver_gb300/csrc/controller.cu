@@ -834,6 +834,7 @@ SolveResult solve_fixed_rbgk(const DeviceOperator& op, const double* d_b, const 
     Statistics stats;
     Workspace ws(op, d_b, reg, o.maximum_basis_size, stream, o.time_operators,
                  o.use_graphs && op.graph_safe(), o.reduced_basis, resident_sms(o));
+    ws.allow_narrow_levels();
     Evaluator ev(ws, op, d_b, reg, stats, stream);
     long long seen[4] = {0, 0, 0, 0};
     auto absorb = [&] {

@@ -1386,7 +1386,10 @@ void Workspace::release() noexcept {
     stream_free(d_carry_, stream_);
     stream_free(d_pwork_, stream_);
     stream_free(d_y_, stream_);
+    stream_free(level_, stream_);
     for (cudaEvent_t e : ev_)
+        if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : nev_)
         if (e) cudaEventDestroy(e);
 }
 

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "device_operator.hpp"
+#include "narrow_block.hpp"
 #include "resident_levels.hpp"
 #include "vector_ops.hpp"
 #include "workspace_state.hpp"
@@ -97,6 +98,15 @@ public:
     const StepAudit& last_step_audit() const { return host_.audit; }
     const DevState& state() const { return host_; }
 
+    // Whether block levels may run as one chain of device work (narrow_block.hpp).
+    // solve_fixed_rbgk asks for it.  AMFLS does not yet: its width controller,
+    // and every policy trained on its decisions, weighs widening by what the
+    // rank-revealing block levels cost (2.4 ms), and with levels of 0.35 ms the
+    // choices a policy has learned no longer gain anything on the study's
+    // dense family (seven held-out solves 0.35 s under the heuristic, 0.45 s
+    // under a policy trained on them).
+    void allow_narrow_levels() { narrow_levels_ = true; }
+
     // Projected solve (krylov_workspace.cpp:833-909): enqueues the candidate
     // x = V y into d_x (n).
     void solve_projected(double* d_x);
@@ -147,8 +157,18 @@ private:
         const double* mat;
         int cols;
     };
+    // A block whose projection passes have already run: whether their
+    // coefficients were finite, and their sums.
+    struct Projected {
+        bool finite;
+        std::vector<double> coefficients;
+    };
     Factor orthogonalize_and_factor(double* block, int cols, const Basis& basis, int max_rank,
-                                    double scale, int tracked, bool retain, double* q_out);
+                                    double scale, int tracked, bool retain, double* q_out,
+                                    const Projected* projected = nullptr);
+    bool narrow_level(int cw, int aw, int max_right, int old_left, narrow::LevelResult* out);
+    double narrow_seconds(int half);
+    Factor narrow_factor(const narrow::Factorisation& f, int cols, int basis_cols);
     bool block_level();
     void enter_block_mode();
     void ensure_block_capacity(int width);
@@ -282,6 +302,9 @@ private:
     int* dflags_ = nullptr;    // [0] nonfinite coefficients, [1] Cholesky, [2] projected
     NormResult* dnorm_ = nullptr;
     cudaEvent_t ev_[2] = {nullptr, nullptr};
+    bool narrow_levels_ = false;
+    narrow::LevelResult* level_ = nullptr;  // of the level in flight
+    cudaEvent_t nev_[4] = {};
 };
 
 // Times the width-one reorthogonalisation sweeps (c = V^T r and the
