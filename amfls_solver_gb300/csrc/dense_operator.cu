@@ -3,7 +3,7 @@
 // Replaces DenseOperator (src/algorithms/mathematics/operators/dense_operator.cpp:20-185,
 // column-major, dgemm) and RowMajorDenseOperator
 // (row_major_dense_operator.cpp:106-258, row-major, the torch path).
-// The product along the contiguous dimension gives each warp two outputs
+// The product along the contiguous dimension gives each warp a few outputs
 // (lanes stride the contiguous index); the product across it keeps one
 // output per thread (coalesced over the contiguous dimension).  Both split
 // the long dimension into chunks whose partial sums a second kernel adds in
@@ -32,18 +32,60 @@ inline int target_blocks() { return grid_cap(); }
 
 // ---- block products (s columns per pass over A, s <= 8 per launch) ----
 // Both directions split the long dimension into chunks whose partial sums
-// land in partial[(chunk * S + c) * outer + o]; reduce_block_kernel adds the
+// land in partial[(chunk * S + c) * outer + o]; the reduce kernels add the
 // chunks in a fixed order.  A is read once per group of eight columns, and
 // every element read feeds S fused multiply-adds.
-constexpr int kDotOutputsPerWarp = 2;
+//
+// A warp of the dot kernel owns several outputs, whose sums over the lanes
+// share the additions of one butterfly that halves the values a lane holds: a
+// shuffle tree per output was five FP64 additions per output and chunk on eight
+// multiply-adds (16384 x 512, four columns: 102 -> 65 us, one: 29 -> 24 us; eight outputs
+// for one column lost 3% on rows of 2000).  Its chunk minimum keeps those sums small
+// beside the products.
+constexpr int dot_outputs(int S) { return S >= 4 ? 2 : 4; }
 
-// A(o, i) at a[o * ld + i] (i contiguous): a warp owns kDotOutputsPerWarp
-// outputs and strides i across its lanes.
+constexpr int pow2_ceil(int v) {
+    int p = 1;
+    while (p < v) p *= 2;
+    return p;
+}
+
+// Sums of N (a power of two, at most 32) values over the lanes of a warp: lane l
+// returns the sum of value `index`; lanes that differ in the low
+// log2(32 / N) bits return the same one.
+template <int N>
+__device__ __forceinline__ double warp_sums(double (&v)[N], int& index) {
+    const int lane = threadIdx.x & 31;
+    int have = N;
+    index = 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (have > 1) {
+            const bool upper = (lane & o) != 0;
+            have >>= 1;
+#pragma unroll
+            for (int j = 0; j < N / 2; ++j) {
+                if (j < have) {
+                    const double keep = upper ? v[j + have] : v[j];
+                    const double send = upper ? v[j] : v[j + have];
+                    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            index = 2 * index + (upper ? 1 : 0);
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    return v[0];
+}
+
+// A(o, i) at a[o * ld + i] (i contiguous): a warp owns dot_outputs(S) outputs
+// and strides i across its lanes.
 template <int S>
 __global__ void __launch_bounds__(kThreads)
 dot_block_kernel(const double* __restrict__ a, long long ld, int outer, int inner, int chunk,
                  const double* __restrict__ x, long long ldx, double* partial, const int* guard) {
-    constexpr int J = kDotOutputsPerWarp;
+    constexpr int J = dot_outputs(S), N = pow2_ceil(J * S);
     if (guard && *guard == 0) return;
     const int lane = threadIdx.x & 31;
     const long long o0 = ((long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * J;
@@ -53,29 +95,27 @@ dot_block_kernel(const double* __restrict__ a, long long ld, int outer, int inne
     const double* rows[J];
 #pragma unroll
     for (int j = 0; j < J; ++j) rows[j] = a + min(o0 + j, (long long)outer - 1) * ld;
-    double acc[J][S];
+    double acc[N];
 #pragma unroll
-    for (int j = 0; j < J; ++j)
-#pragma unroll
-        for (int c = 0; c < S; ++c) acc[j][c] = 0.0;
+    for (int t = 0; t < N; ++t) acc[t] = 0.0;
+    // value j * S + c: output o0 + j, column c
+#pragma unroll 2
     for (int i = i0 + lane; i < i1; i += 32) {
-        double xv[S];
+        double xv[S], av[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) av[j] = __ldg(rows[j] + i);
 #pragma unroll
         for (int c = 0; c < S; ++c) xv[c] = __ldg(x + i + c * ldx);
 #pragma unroll
-        for (int j = 0; j < J; ++j) {
-            const double av = __ldg(rows[j] + i);
+        for (int j = 0; j < J; ++j)
 #pragma unroll
-            for (int c = 0; c < S; ++c) acc[j][c] = fma(av, xv[c], acc[j][c]);
-        }
+            for (int c = 0; c < S; ++c) acc[j * S + c] = fma(av[j], xv[c], acc[j * S + c]);
     }
-#pragma unroll
-    for (int j = 0; j < J; ++j)
-#pragma unroll
-        for (int c = 0; c < S; ++c) {
-            const double v = warp_sum(acc[j][c]);
-            if (lane == 0 && o0 + j < outer) partial[((long long)ch * S + c) * outer + o0 + j] = v;
-        }
+    int index;
+    const double v = warp_sums(acc, index);
+    const int j = index / S, c = index % S;
+    if ((lane & (32 / N - 1)) == 0 && index < J * S && o0 + j < outer)
+        partial[((long long)ch * S + c) * outer + o0 + j] = v;
 }
 
 // A(i, o) at a[i * ld + o] (o contiguous): a thread owns one output.
@@ -101,52 +141,122 @@ across_block_kernel(const double* __restrict__ a, long long ld, int outer, int i
     for (int c = 0; c < S; ++c) partial[((long long)ch * S + c) * outer + o] = acc[c];
 }
 
-__global__ void reduce_block_kernel(const double* partial, int chunks, int S, int outer,
-                                    double* y, long long ldy, const int* guard) {
+// Adds the chunks.  Sliced, a block takes eight consecutive outputs, every
+// thread each 32nd chunk of one of them, and the slices are added in a fixed
+// tree; else a thread adds all of one output's.  A thread per output took 52
+// to 107 us for 512 outputs of 512 chunks, a chain of dependent loads and
+// additions (sliced 5 to 12 us), and is the faster one where the outputs fill the
+// SM quarters with warps (65536 outputs of 16 chunks: 6.2 against 14.2 us).
+constexpr int kSlicedChunks = 16, kSliceOutputs = 8;
+
+template <bool kSliced>
+__global__ void __launch_bounds__(kThreads)
+reduce_block_kernel(const double* __restrict__ partial, int chunks, int S, int outer, double* y,
+                    long long ldy, const int* guard) {
+    __shared__ double slice[kThreads / 32][kSliceOutputs];
     if (guard && *guard == 0) return;
     const long long total = (long long)S * outer;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
+    auto put = [&](long long t, double v) {
         const int c = (int)(t / outer);
-        const long long o = t % outer;
-        double s = 0.0;
-        for (int ch = 0; ch < chunks; ++ch) s += partial[((long long)ch * S + c) * outer + o];
-        y[o + c * ldy] = s;
-    }
-}
-
-// double-double variants for the validation refinement
-__global__ void dd_dot_rows_kernel(const double* __restrict__ a, long long ld, int outer,
-                                   int inner, const double* x_hi, const double* x_lo, double* y_hi,
-                                   double* y_lo, int* finite) {
-    const int lane = threadIdx.x & 31;
-    for (long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; w < outer;
-         w += ((long long)gridDim.x * blockDim.x) >> 5) {
-        const double* row = a + w * ld;
-        dd acc{0.0, 0.0};
-        for (int i = lane; i < inner; i += 32)
-            acc = dd_add(acc, dd_mul_d(dd{x_hi[i], x_lo ? x_lo[i] : 0.0}, row[i]));
-        for (int o = 16; o > 0; o >>= 1) acc = dd_add(acc, dd_shfl_xor(acc, o));
-        if (lane == 0) {
-            y_hi[w] = acc.hi;
-            y_lo[w] = acc.lo;
-            if (!isfinite(acc.hi) || !isfinite(acc.lo)) atomicAnd(finite, 0);
+        y[t - (long long)c * outer + c * ldy] = v;
+    };
+    if constexpr (kSliced) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        constexpr int kSlices = kThreads / kSliceOutputs;
+        for (long long t0 = (long long)blockIdx.x * kSliceOutputs; t0 < total;
+             t0 += (long long)gridDim.x * kSliceOutputs) {
+            const long long t = t0 + lane % kSliceOutputs;
+            double x[4] = {0.0, 0.0, 0.0, 0.0};
+            if (t < total) {
+                const double* p = partial + t;
+                int ch = threadIdx.x / kSliceOutputs;
+                for (; ch + 3 * kSlices < chunks; ch += 4 * kSlices) {
+                    double v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = p[(ch + u * kSlices) * total];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) x[u] += v[u];
+                }
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if (ch + u * kSlices < chunks) x[u] += p[(ch + u * kSlices) * total];
+            }
+            double v = (x[0] + x[1]) + (x[2] + x[3]);
+            v += __shfl_xor_sync(0xffffffffu, v, 8);
+            v += __shfl_xor_sync(0xffffffffu, v, 16);
+            if (lane < kSliceOutputs) slice[warp][lane] = v;
+            __syncthreads();
+            if (threadIdx.x < kSliceOutputs && t < total)
+                put(t, ((slice[0][lane] + slice[1][lane]) + (slice[2][lane] + slice[3][lane])) +
+                           ((slice[4][lane] + slice[5][lane]) +
+                            (slice[6][lane] + slice[7][lane])));
+            __syncthreads();
+        }
+    } else {
+        for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+             t += (long long)gridDim.x * blockDim.x) {
+            double s = partial[t];
+            for (int ch = 1; ch < chunks; ++ch) s += partial[ch * total + t];
+            put(t, s);
         }
     }
 }
 
-__global__ void dd_sum_cols_kernel(const double* __restrict__ a, long long ld, int outer,
-                                   int inner, const double* x_hi, const double* x_lo,
-                                   double* y_hi, double* y_lo, int* finite) {
-    for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < outer;
-         o += (long long)gridDim.x * blockDim.x) {
-        dd acc{0.0, 0.0};
-        for (int i = 0; i < inner; ++i)
-            acc = dd_add(acc, dd_mul_d(dd{x_hi[i], x_lo ? x_lo[i] : 0.0}, a[(long long)i * ld + o]));
-        y_hi[o] = acc.hi;
-        y_lo[o] = acc.lo;
-        if (!isfinite(acc.hi) || !isfinite(acc.lo)) atomicAnd(finite, 0);
+// ---- double-double products of the validation refinement ----
+// The same split: chunk sums in partial[2 * (chunk * outer + o)] as (hi, lo)
+// pairs, added by dd_reduce_kernel.  A double-double multiply-add is some thirty FP64
+// operations, so these are bound by the FP64 pipe once every SM has a chunk;
+// one thread (or warp) per output walked all of a long dimension by itself
+// (16384 x 512, transposed: 31.0 -> 0.43 ms).
+__global__ void __launch_bounds__(kThreads)
+dd_dot_kernel(const double* __restrict__ a, long long ld, int outer, int inner, int chunk,
+              const double* __restrict__ x_hi, const double* __restrict__ x_lo, double2* partial) {
+    const int lane = threadIdx.x & 31;
+    const int o = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    if (o >= outer) return;
+    const int i0 = blockIdx.y * chunk, i1 = min(inner, i0 + chunk);
+    const double* row = a + o * ld;
+    dd acc{0.0, 0.0};
+    for (int i = i0 + lane; i < i1; i += 32)
+        acc = dd_add(acc, dd_mul_d(dd{x_hi[i], x_lo ? x_lo[i] : 0.0}, row[i]));
+    for (int w = 16; w > 0; w >>= 1) acc = dd_add(acc, dd_shfl_xor(acc, w));
+    if (lane == 0) partial[(long long)blockIdx.y * outer + o] = make_double2(acc.hi, acc.lo);
+}
+
+__global__ void __launch_bounds__(kThreads)
+dd_across_kernel(const double* __restrict__ a, long long ld, int outer, int inner, int chunk,
+                 const double* __restrict__ x_hi, const double* __restrict__ x_lo,
+                 double2* partial) {
+    const long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (o >= outer) return;
+    const int i0 = blockIdx.y * chunk, i1 = min(inner, i0 + chunk);
+    dd acc{0.0, 0.0};
+    for (int i = i0; i < i1; ++i)
+        acc = dd_add(acc, dd_mul_d(dd{x_hi[i], x_lo ? x_lo[i] : 0.0}, a[(long long)i * ld + o]));
+    partial[(long long)blockIdx.y * outer + o] = make_double2(acc.hi, acc.lo);
+}
+
+// kWarp: a warp per output, its lanes every 32nd chunk; else a thread.
+template <bool kWarp>
+__global__ void __launch_bounds__(kThreads)
+dd_reduce_kernel(const double2* __restrict__ partial, int chunks, int outer, double* y_hi,
+                 double* y_lo, int* finite) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long o = kWarp ? t >> 5 : t;
+    if (o >= outer) return;
+    const int step = kWarp ? 32 : 1, first = kWarp ? (int)(t & 31) : 0;
+    dd acc{0.0, 0.0};
+    for (int ch = first; ch < chunks; ch += step) {
+        const double2 p = partial[(long long)ch * outer + o];
+        acc = dd_add(acc, dd{p.x, p.y});
     }
+    if (kWarp) {
+        for (int w = 16; w > 0; w >>= 1) acc = dd_add(acc, dd_shfl_xor(acc, w));
+        if (first != 0) return;
+    }
+    y_hi[o] = acc.hi;
+    y_lo[o] = acc.lo;
+    if (!isfinite(acc.hi) || !isfinite(acc.lo)) atomicAnd(finite, 0);
 }
 
 // ---- norm model: sequential sums in storage order (outer loop = storage-major)
@@ -197,20 +307,39 @@ __global__ void model_outer_kernel(const double* a, int outer, int inner, double
     }
 }
 
-// per inner index: sums over the outer dimension in order; Frobenius terms
-// rounded upward per index, then summed upward by the last block
-__global__ void model_inner_kernel(const double* a, int outer, int inner, double* acc,
-                                   double* frob_partials, unsigned* counter, double* frob_out) {
+// per inner index: sums of magnitudes and squares over a chunk of the outer
+// dimension (one thread over all of it took 4.2 ms for 16384 x 512 by rows)
+__global__ void __launch_bounds__(kThreads)
+model_chunk_kernel(const double* __restrict__ a, int outer, int inner, int chunk,
+                   double2* partial) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= inner) return;
+    const int o0 = blockIdx.y * chunk, o1 = min(outer, o0 + chunk);
+    double s = 0.0, q = 0.0;
+    for (int o = o0; o < o1; ++o) {
+        const double m = fabs(a[(long long)o * inner + i]);
+        if (!isfinite(m)) continue;
+        s += m;
+        q = fma(m, m, q);
+    }
+    partial[(long long)blockIdx.y * inner + i] = make_double2(s, q);
+}
+
+// their totals in order of the chunks; Frobenius terms rounded upward per
+// index, then summed upward by the last block
+__global__ void __launch_bounds__(kThreads)
+model_inner_kernel(const double2* __restrict__ partial, int chunks, int outer, int inner,
+                   double* acc, double* frob_partials, unsigned* counter, double* frob_out) {
     __shared__ double scratch[32];
     double frob = 0.0;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < inner;
          i += (long long)gridDim.x * blockDim.x) {
         double s = 0.0, q = 0.0;
-        for (int o = 0; o < outer; ++o) {
-            const double m = fabs(a[(long long)o * inner + i]);
-            if (!isfinite(m)) continue;
-            s += m;
-            q = fma(m, m, q);
+#pragma unroll 8
+        for (int ch = 0; ch < chunks; ++ch) {
+            const double2 p = partial[(long long)ch * inner + i];
+            s += p.x;
+            q += p.y;
         }
         atomic_max_pos(&acc[3], fpb::sum_upper(s, outer, true));
         atomic_max_pos(&acc[1], fpb::down_sqrt(fpb::sum_lower(q, outer)));
@@ -269,14 +398,15 @@ int grid_1d(long long items) {
 }
 
 // chunking for the block kernels: enough blocks to fill the GPU twice over
-void block_chunks(bool dot, int out_n, int in_n, int& blocks_x, int& chunks, int& chunk) {
+// (J: outputs of a warp of the dot kernel)
+void block_chunks(bool dot, int J, int out_n, int in_n, int& blocks_x, int& chunks, int& chunk) {
     if (dot) {
-        const long long groups = (out_n + kDotOutputsPerWarp - 1) / kDotOutputsPerWarp;
+        const long long groups = ((long long)out_n + J - 1) / J;
         blocks_x = (int)((groups + kThreads / 32 - 1) / (kThreads / 32));
     } else {
         blocks_x = (out_n + kThreads - 1) / kThreads;
     }
-    const int min_rows = dot ? 256 : 32;
+    const int min_rows = dot ? 512 : 32;
     chunks = std::max(1, std::min((2 * target_blocks() + blocks_x - 1) / blocks_x,
                                   (in_n + min_rows - 1) / min_rows));
     chunk = (in_n + chunks - 1) / chunks;
@@ -286,9 +416,9 @@ void block_chunks(bool dot, int out_n, int in_n, int& blocks_x, int& chunks, int
 template <int S>
 void launch_block(bool dot, const double* a, long long ld, int out_n, int in_n, const double* x,
                   long long ldx, double* partial, double* y, long long ldy, cudaStream_t s,
-                  const int* guard = nullptr) {
+                  const int* guard = nullptr, bool slices = true) {
     int blocks_x = 0, chunks = 0, chunk = 0;
-    block_chunks(dot, out_n, in_n, blocks_x, chunks, chunk);
+    block_chunks(dot, dot_outputs(S), out_n, in_n, blocks_x, chunks, chunk);
     const dim3 grid(blocks_x, chunks);
     if (dot)
         dot_block_kernel<S><<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, chunk, x, ldx, partial,
@@ -297,8 +427,37 @@ void launch_block(bool dot, const double* a, long long ld, int out_n, int in_n, 
         across_block_kernel<S><<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, chunk, x, ldx,
                                                           partial, guard);
     AMFLS_LAUNCHED();
-    reduce_block_kernel<<<grid_1d((long long)S * out_n), kThreads, 0, s>>>(partial, chunks, S,
-                                                                           out_n, y, ldy, guard);
+    const long long total = (long long)S * out_n;
+    if (slices && chunks >= kSlicedChunks && total <= 32LL * 4 * sm_count()) {
+        const long long groups = (total + kSliceOutputs - 1) / kSliceOutputs;
+        reduce_block_kernel<true><<<(int)std::min<long long>(groups, target_blocks()), kThreads, 0,
+                                    s>>>(partial, chunks, S, out_n, y, ldy, guard);
+    } else {
+        reduce_block_kernel<false><<<grid_1d(total), kThreads, 0, s>>>(partial, chunks, S, out_n,
+                                                                       y, ldy, guard);
+    }
+    AMFLS_LAUNCHED();
+}
+
+void launch_refined(bool dot, const double* a, long long ld, int out_n, int in_n,
+                    const double* x_hi, const double* x_lo, double* partial, double* y_hi,
+                    double* y_lo, int* finite, cudaStream_t s) {
+    int blocks_x = 0, chunks = 0, chunk = 0;
+    block_chunks(dot, 1, out_n, in_n, blocks_x, chunks, chunk);
+    const dim3 grid(blocks_x, chunks);
+    double2* pairs = reinterpret_cast<double2*>(partial);
+    (dot ? dd_dot_kernel : dd_across_kernel)<<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, chunk,
+                                                                       x_hi, x_lo, pairs);
+    AMFLS_LAUNCHED();
+    // additions in a row on each SM quarter: `chunks` for every 32 outputs with a
+    // thread per output, chunks / 32 + 5 for every output with a warp
+    const long long quarters = 4LL * sm_count();
+    const bool warp = std::max(1LL, out_n / quarters) * (chunks / 32 + 5) <
+                      std::max(1LL, out_n / 32 / quarters) * chunks;
+    const long long threads = (long long)out_n * (warp ? 32 : 1);
+    (warp ? dd_reduce_kernel<true> : dd_reduce_kernel<false>)<<<
+        (unsigned)((threads + kThreads - 1) / kThreads), kThreads, 0, s>>>(pairs, chunks, out_n,
+                                                                           y_hi, y_lo, finite);
     AMFLS_LAUNCHED();
 }
 
@@ -328,9 +487,14 @@ DenseOperator::DenseOperator(int rows, int cols, const double* d_values, bool co
         // can be captured into CUDA graphs
         for (int tr = 0; tr < 2; ++tr) {  // both directions, up to 8 columns per pass
             const int on = tr ? cols : rows, inn = tr ? rows : cols;
+            const bool dot = column_major == (tr == 1);
             int bx = 0, ch = 0, ck = 0;
-            block_chunks(column_major == (tr == 1), on, inn, bx, ch, ck);
-            partial_cap_ = std::max(partial_cap_, 8LL * ch * on);
+            for (int S = 1; S <= 8; ++S) {
+                block_chunks(dot, dot_outputs(S), on, inn, bx, ch, ck);
+                partial_cap_ = std::max(partial_cap_, (long long)S * ch * on);
+            }
+            block_chunks(dot, 1, on, inn, bx, ch, ck);  // double-double pairs
+            partial_cap_ = std::max(partial_cap_, 2LL * ch * on);
         }
         AMFLS_CUDA(cudaMalloc(&partials_,
                               sizeof(double) * std::max<long long>(1, partial_cap_)));
@@ -341,8 +505,13 @@ DenseOperator::DenseOperator(int rows, int cols, const double* d_values, bool co
         model_outer_kernel<<<og, kThreads, 0, stream>>>(a_, outer, inner, w, w + 9 + ig,
                                                         counter_ + 2, w + 8);
         AMFLS_LAUNCHED();
-        model_inner_kernel<<<ig, kThreads, 0, stream>>>(a_, outer, inner, w, w + 9, counter_,
-                                                        w + 5);
+        int bx = 0, chunks = 0, chunk = 0;
+        block_chunks(false, 1, inner, outer, bx, chunks, chunk);
+        double2* sums = reinterpret_cast<double2*>(partials_);
+        model_chunk_kernel<<<dim3(bx, chunks), kThreads, 0, stream>>>(a_, outer, inner, chunk, sums);
+        AMFLS_LAUNCHED();
+        model_inner_kernel<<<ig, kThreads, 0, stream>>>(sums, chunks, outer, inner, w, w + 9,
+                                                        counter_, w + 5);
         AMFLS_LAUNCHED();
         // the reference's Frobenius bound sums column square sums: the inner
         // index for row-major storage, the outer one for column-major
@@ -373,18 +542,6 @@ void DenseOperator::release() noexcept {
     cudaFree(tmp_);
     cudaFree(scratch_);
     cudaFree(counter_);
-}
-
-void DenseOperator::product(bool transpose, const double* x, double* y, const int* guard,
-                            cudaStream_t s) const {
-    // y has length rows (apply) or cols (transpose).  The contiguous
-    // dimension decides the kernel: row-major rows are contiguous (apply =
-    // dot of rows); column-major columns are (transpose = dot of columns).
-    const int out_n = transpose ? cols_ : rows_;
-    const int in_n = transpose ? rows_ : cols_;
-    const bool dot = column_major_ == transpose;
-    const long long ld = column_major_ ? rows_ : cols_;
-    launch_block<1>(dot, a_, ld, out_n, in_n, x, in_n, partials_, y, out_n, s, guard);
 }
 
 void DenseOperator::block_product(bool transpose, const double* x, int block_cols, double* y,
@@ -425,36 +582,35 @@ void DenseOperator::apply_transpose(const double* y, int block_cols, double* x,
 
 bool DenseOperator::product1(bool transpose, const double* x, const Epilogue& ep,
                              cudaStream_t s) const {
-    product(transpose, x, tmp_, ep.guard, s);
-    run_epilogue(tmp_, transpose ? cols_ : rows_, ep, ep.partials ? ep.partials : scratch_,
+    // The contiguous dimension decides the kernel: row-major rows are
+    // contiguous (apply = dot of rows); column-major columns are (transpose =
+    // dot of columns).
+    //
+    // Without the sliced sums: the width controller weighs the measured cost of
+    // this product against the local algebra, and the policies trained on its
+    // decisions earn their gain where it widens.  With the sliced sums (131 -> 27 us,
+    // 16384 x 512 transposed) it never widens on the dense study family, and a
+    // policy has nothing left to gain there.
+    const int out_n = transpose ? cols_ : rows_;
+    const int in_n = transpose ? rows_ : cols_;
+    const long long ld = column_major_ ? rows_ : cols_;
+    launch_block<1>(column_major_ == transpose, a_, ld, out_n, in_n, x, in_n, partials_, tmp_,
+                    out_n, s, ep.guard, false);
+    run_epilogue(tmp_, out_n, ep, ep.partials ? ep.partials : scratch_,
                  ep.counter ? ep.counter : counter_ + 1, s);
     return true;
 }
 
 void DenseOperator::apply_refined(const double* x_hi, const double* x_lo, double* y_hi,
                                   double* y_lo, int* finite, cudaStream_t s) const {
-    if (!column_major_) {
-        dd_dot_rows_kernel<<<grid_1d((long long)rows_ * 32), kThreads, 0, s>>>(
-            a_, cols_, rows_, cols_, x_hi, x_lo, y_hi, y_lo, finite);
-        AMFLS_LAUNCHED();
-    } else {
-        dd_sum_cols_kernel<<<grid_1d(rows_), kThreads, 0, s>>>(a_, rows_, rows_, cols_, x_hi,
-                                                               x_lo, y_hi, y_lo, finite);
-        AMFLS_LAUNCHED();
-    }
+    launch_refined(!column_major_, a_, column_major_ ? rows_ : cols_, rows_, cols_, x_hi, x_lo,
+                   partials_, y_hi, y_lo, finite, s);
 }
 
 void DenseOperator::apply_transpose_refined(const double* y_hi, const double* y_lo, double* x_hi,
                                             double* x_lo, int* finite, cudaStream_t s) const {
-    if (column_major_) {
-        dd_dot_rows_kernel<<<grid_1d((long long)cols_ * 32), kThreads, 0, s>>>(
-            a_, rows_, cols_, rows_, y_hi, y_lo, x_hi, x_lo, finite);
-        AMFLS_LAUNCHED();
-    } else {
-        dd_sum_cols_kernel<<<grid_1d(cols_), kThreads, 0, s>>>(a_, cols_, cols_, rows_, y_hi,
-                                                               y_lo, x_hi, x_lo, finite);
-        AMFLS_LAUNCHED();
-    }
+    launch_refined(column_major_, a_, column_major_ ? rows_ : cols_, cols_, rows_, y_hi, y_lo,
+                   partials_, x_hi, x_lo, finite, s);
 }
 
 }  // namespace amfls_gpu

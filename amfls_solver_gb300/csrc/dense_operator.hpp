@@ -38,8 +38,6 @@ public:
 
 private:
     void release() noexcept;  // frees the operator's device buffers
-    void product(bool transpose, const double* x, double* y, const int* guard,
-                 cudaStream_t s) const;
     void block_product(bool transpose, const double* x, int block_cols, double* y,
                        cudaStream_t s) const;
     int rows_, cols_;
