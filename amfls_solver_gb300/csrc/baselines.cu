@@ -6,7 +6,10 @@
 // vectors stay on the device (products through the operator, elementwise
 // updates and norms as kernels), and every checkpoint of the reference's
 // CertificateCheckpointSchedule certifies the current iterate with the
-// device validation, exactly where the reference validates.  The norms are
+// device validation, exactly where the reference validates.  On CSR operators
+// the iterations in between run as one kernel with the recurrences on the
+// device (resident_baselines.cu), and the host steps below take what that
+// kernel hands back: breakdowns and values out of range.  The norms are
 // the scaled two-pass norms that stand in for dnrm2 elsewhere in the
 // library, and the vector updates contract to FMAs, so iterates agree with
 // the reference's to rounding rather than bit for bit.
@@ -20,6 +23,7 @@
 
 #include "baselines.hpp"
 #include "common.cuh"
+#include "resident_baselines.hpp"
 #include "solve_common.hpp"
 #include "validation.hpp"
 #include "vector_ops.hpp"
@@ -125,6 +129,20 @@ public:
         ++stats.search_at_columns;
         ++stats.search_at_block_calls;
     }
+    // search products that ran inside a resident kernel
+    void count_products(long long a, long long at, double a_s, double at_s) {
+        stats.a_columns += a;
+        stats.a_block_calls += a;
+        stats.search_a_columns += a;
+        stats.search_a_block_calls += a;
+        stats.at_columns += at;
+        stats.at_block_calls += at;
+        stats.search_at_columns += at;
+        stats.search_at_block_calls += at;
+        stats.a_seconds += a_s;
+        stats.at_seconds += at_s;
+    }
+    cudaStream_t stream() const { return s_; }
     Statistics stats;
 
 private:
@@ -192,6 +210,11 @@ public:
         return v_;
     }
     bool should_evaluate(int it) const { return sched_.should_evaluate(it); }
+    // the next iteration after `it` that is certified, max_it at the latest
+    int next(int it, int max_it) const {
+        for (++it; it < max_it && !sched_.should_evaluate(it);) ++it;
+        return it;
+    }
     bool failed() const { return failed_numerically(v_); }
     bool success() const { return status_ == 0; }
     void set_outcome(int status, int reason) {
@@ -222,6 +245,64 @@ private:
     SolveResult out_;
     ValidationOutput v_{};
     int it_ = 0, status_ = 1, reason_ = 3;
+};
+
+// The resident iterations of one solve; unavailable without the operator's
+// tables.
+class Resident {
+public:
+    Resident(const DeviceOperator& op, Run& run, bool lsmr, double damp)
+        : run_(run), lsmr_(lsmr) {
+        ResidentOperator view;
+        if (!op.resident(&view) || view.augmented) return;
+        grid_ = sm_count();
+        args_.a = view.a;
+        args_.t = view.t;
+        args_.m = view.rows;
+        args_.n = view.cols;
+        args_.damp = damp;
+        args_.left = run.vec(view.rows);
+        args_.right = run.vec(view.cols);
+        args_.red = run.vec(2LL * 4 * grid_);
+        static_assert(sizeof(BaselineState) % sizeof(double) == 0);
+        args_.st = reinterpret_cast<BaselineState*>(
+            run.vec(sizeof(BaselineState) / sizeof(double)));
+        args_.barrier = reinterpret_cast<unsigned*>(run.vec(1));
+    }
+    bool available() const { return grid_ > 0; }
+    BaselineArgs& args() { return args_; }
+    // Takes half-steps from p until `target` are done (true) or one is handed
+    // back (false: p is where the general path goes on).  p's indices say which of
+    // each pair of vectors is the current one afterwards.
+    bool advance(BaselinePosition& p, int target) {
+        const int from = p.pos;
+        p.u = p.v = 0;
+        BaselineState st{};
+        st.now = p;
+        st.target = target;
+        const cudaStream_t s = run_.stream();
+        lease_.acquire(grid_);
+        put(args_.st, st, s);
+        AMFLS_CUDA(cudaMemsetAsync(args_.barrier, 0, sizeof(unsigned), s));
+        launch_resident_baseline(args_, lsmr_, grid_, s);
+        read_back(&st, args_.st, s);
+        lease_.release();
+        if (st.timeout) throw std::runtime_error("resident iterations: a grid barrier timed out");
+        const bool reached = !st.handed_back && !st.nonfinite[0] && !st.nonfinite[1];
+        p = reached || st.handed_back ? st.now : st.back;
+        // half-steps 2i are A's, 2i + 1 A^T's
+        run_.count_products((p.pos + 1) / 2 - (from + 1) / 2, p.pos / 2 - from / 2,
+                            1e-9 * st.a_ns, 1e-9 * st.at_ns);
+        if (!reached && p.pos == from) grid_ = 0;  // no progress: leave it to the general path
+        return reached;
+    }
+
+private:
+    Run& run_;
+    bool lsmr_;
+    int grid_ = 0;
+    BaselineArgs args_{};
+    SmLease lease_;
 };
 
 bool finite_all(std::initializer_list<double> values) {
@@ -255,6 +336,8 @@ SolveResult solve_lsqr(const DeviceOperator& op, const double* d_b, const Baseli
     double* atu = run.vec(n);
     double* w = run.vec(n);
     double* x = run.vec(n);
+    double* nw = run.vec(n);
+    double* nx = run.vec(n);
 
     run.copy(u, d_b, m);
     NormResult nr = run.norms({{u, m}});
@@ -275,36 +358,57 @@ SolveResult solve_lsqr(const DeviceOperator& op, const double* d_b, const Baseli
         if (cand.failed() || cand.success() || alpha == 0.0)
             return cand.finish(x, d_solution, t0, launches0, stream);
     }
-    for (int it = 1; it <= max_it; ++it) {
-        run.apply(v, av);
-        run.combine(av, av, -alpha, u, m);
-        beta = euclid_from(run.norms({{av, m}}), 0);
-        if (beta > 0.0) run.scale(av, 1.0 / beta, m);
-
-        // x_k needs beta_{k+1} only: it is formed (and certified at a
-        // checkpoint) before the transpose half-step
-        const double rhobar1 = std::hypot(rhobar, damp);
-        const double cs1 = rhobar1 == 0.0 ? 1.0 : rhobar / rhobar1;
-        phibar *= cs1;
-        const double rho = std::hypot(rhobar1, beta);
-        const double cs = rho == 0.0 ? 1.0 : rhobar1 / rho;
-        const double sn = rho == 0.0 ? 0.0 : beta / rho;
-        const double phi = cs * phibar;
-        phibar = sn * phibar;
-        bool finite = finite_all({beta, rhobar1, cs1, rho, cs, sn, phi, phibar});
-        if (rho != 0.0) {
-            const double update = phi / rho;
-            finite = finite && std::isfinite(update);
-            run.combine(x, x, update, w, n);
+    Resident device(op, run, false, damp);
+    double rho = 0.0, cs = 1.0, sn = 0.0;
+    int evaluated = 0;  // the last certified iteration
+    // half-steps done: A's in 2i, A^T's in 2i + 1
+    for (int pos = 0; pos < 2 * max_it;) {
+        bool finite = true, breakdown = false, at_iterate = false;
+        if (device.available()) {
+            BaselineArgs& g = device.args();
+            g.u[0] = u, g.u[1] = av, g.v[0] = v, g.v[1] = atu;
+            g.x[0] = x, g.x[1] = nx, g.w[0] = w, g.w[1] = nw;
+            BaselinePosition p{};
+            p.alpha = alpha, p.beta = beta, p.rho = rho, p.rhobar = rhobar;
+            p.cbar = cs, p.sbar = sn, p.zetabar = phibar, p.pos = pos;
+            at_iterate = device.advance(p, 2 * cand.next((pos + 1) / 2, max_it) - 1);
+            alpha = p.alpha, beta = p.beta, rho = p.rho, rhobar = p.rhobar;
+            cs = p.cbar, sn = p.sbar, phibar = p.zetabar, pos = p.pos;
+            if (p.u) std::swap(u, av), std::swap(x, nx);
+            if (p.v) std::swap(v, atu), std::swap(w, nw);
         }
-        finite = finite && run.norms({{x, n}}).nonfinite[0] == 0;
-        std::swap(u, av);
+        if (!at_iterate && pos % 2 == 0) {
+            run.apply(v, av);
+            run.combine(av, av, -alpha, u, m);
+            beta = euclid_from(run.norms({{av, m}}), 0);
+            if (beta > 0.0) run.scale(av, 1.0 / beta, m);
 
-        const bool breakdown = beta == 0.0;
-        bool evaluated = false;
-        if (cand.should_evaluate(it) || breakdown || !finite || it == max_it) {
+            // x_k needs beta_{k+1} only: it is formed (and certified at a
+            // checkpoint) before the transpose half-step
+            const double rhobar1 = std::hypot(rhobar, damp);
+            const double cs1 = rhobar1 == 0.0 ? 1.0 : rhobar / rhobar1;
+            phibar *= cs1;
+            rho = std::hypot(rhobar1, beta);
+            cs = rho == 0.0 ? 1.0 : rhobar1 / rho;
+            sn = rho == 0.0 ? 0.0 : beta / rho;
+            const double phi = cs * phibar;
+            phibar = sn * phibar;
+            finite = finite_all({beta, rhobar1, cs1, rho, cs, sn, phi, phibar});
+            if (rho != 0.0) {
+                const double update = phi / rho;
+                finite = finite && std::isfinite(update);
+                run.combine(x, x, update, w, n);
+            }
+            finite = finite && run.norms({{x, n}}).nonfinite[0] == 0;
+            std::swap(u, av);
+            breakdown = beta == 0.0;
+            at_iterate = true;
+            ++pos;
+        }
+        const int it = (pos + 1) / 2;
+        if (at_iterate && (cand.should_evaluate(it) || breakdown || !finite || it == max_it)) {
             cand.evaluate(x, it);
-            evaluated = true;
+            evaluated = it;
             if (cand.failed() || cand.success()) break;
             if (!finite) {
                 cand.set_outcome(4, 7);
@@ -319,6 +423,7 @@ SolveResult solve_lsqr(const DeviceOperator& op, const double* d_b, const Baseli
                 break;
             }
         }
+        if (at_iterate && device.available()) continue;  // it takes the transpose half-step
 
         run.apply_transpose(u, atu);
         run.combine(atu, atu, -beta, v, n);
@@ -335,7 +440,7 @@ SolveResult solve_lsqr(const DeviceOperator& op, const double* d_b, const Baseli
             cont = run.norms({{w, n}}).nonfinite[0] == 0;
         }
         if (!cont || next_alpha == 0.0) {
-            if (!evaluated) {
+            if (evaluated != it) {
                 cand.evaluate(x, it);
                 if (cand.failed() || cand.success()) break;
             }
@@ -345,6 +450,7 @@ SolveResult solve_lsqr(const DeviceOperator& op, const double* d_b, const Baseli
         alpha = next_alpha;
         rhobar = next_rhobar;
         std::swap(v, atu);
+        ++pos;
     }
     return cand.finish(x, d_solution, t0, launches0, stream);
 }
@@ -394,7 +500,28 @@ SolveResult solve_lsmr(const DeviceOperator& op, const double* d_b, const Baseli
         if (cand.success() || initial_breakdown || alpha == 0.0)
             return cand.finish(x, d_solution, t0, launches0, stream);
     }
-    for (int it = 1; it <= max_it; ++it) {
+    Resident device(op, run, true, damp);
+    for (int it = 0; it < max_it;) {
+        if (device.available()) {
+            BaselineArgs& g = device.args();
+            g.u[0] = u, g.u[1] = av, g.v[0] = v, g.v[1] = atu, g.x[0] = x, g.x[1] = nx;
+            g.w[0] = h, g.w[1] = nh, g.hbar[0] = hbar, g.hbar[1] = nhbar;
+            BaselinePosition p{};
+            p.alpha = alpha, p.rho = rho, p.rhobar = rhobar, p.cbar = cbar, p.sbar = sbar;
+            p.alphabar = alphabar, p.zetabar = zetabar, p.pos = 2 * it;
+            const bool reached = device.advance(p, 2 * cand.next(it, max_it));
+            alpha = p.alpha, rho = p.rho, rhobar = p.rhobar, cbar = p.cbar, sbar = p.sbar;
+            alphabar = p.alphabar, zetabar = p.zetabar, it = p.pos / 2;
+            if (p.u) std::swap(u, av);
+            if (p.v) std::swap(v, atu), std::swap(x, nx), std::swap(h, nh), std::swap(hbar, nhbar);
+            if (reached) {
+                cand.evaluate(x, it);
+                if (cand.failed() || cand.success()) break;
+                if (it == max_it) cand.set_outcome(1, 3);
+                continue;
+            }
+        }
+        ++it;
         run.apply(v, av);
         bool valid = run.norms({{av, m}}).nonfinite[0] == 0;
         run.combine(av, av, -alpha, u, m);

@@ -45,14 +45,13 @@
 
 #include "common.cuh"
 #include "level_decisions.cuh"
+#include "resident_grid.cuh"
 #include "resident_levels.hpp"
 
 namespace amfls_gpu {
 namespace {
 
-constexpr int kT = kResidentThreads;
-constexpr int kW = kT / 32;
-constexpr unsigned kSpinLimit = 1u << 23;  // polls of about a microsecond
+using namespace resident;
 
 enum Slot { kRedRight = 0, kRedNorm = 1, kRedNorm2 = 2, kRedA = 3, kRedLeft = 4, kRedLeft2 = 5 };
 constexpr int kMaxPanels = kResidentMaxBasis / 32 + 1;
@@ -60,10 +59,8 @@ constexpr int kSlots = 2;           // ring slots of a warp
 constexpr int kSlotBytes = 4096;
 constexpr int kSegs = 4;  // panels of V^T r whose partial sums are added together
 
-struct Shared {
+struct Shared : GridShared<3> {
     DevState st;
-    unsigned arrived;   // barrier arrivals expected so far
-    int failed;
     int left_raw;
     double val[4];      // reduced values
     // shares of the V^T r units for the current number of panels
@@ -73,89 +70,11 @@ struct Shared {
     short seg_first[kMaxPanels], seg_last[kMaxPanels];  // blocks with units of a panel
     double* panels[kMaxPanels];
     alignas(16) double seg[kSegs][kW][32];  // stored and read in pairs
-    double lane[3][kT];
 };
 
 constexpr size_t kSharedBytes = (sizeof(Shared) + 127) / 128 * 128;
 constexpr size_t kRingBytes = (size_t)kW * kSlots * kSlotBytes;
 static_assert(offsetof(Shared, seg) % 16 == 0 && kW <= 16);
-
-// Grid barrier: the block's writes before it are visible to every block after
-// it (the fences of thread 0 are cumulative over the block barriers around
-// them, and the second one drops stale L1 lines).
-__device__ __forceinline__ void grid_barrier(Shared& s, unsigned* bar) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s.arrived += gridDim.x;
-        const unsigned want = s.arrived;
-        __threadfence();
-        atomicAdd(bar, 1u);
-        unsigned seen, spins = 0;
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-            if (++spins > kSpinLimit) {
-                s.failed = 1;
-                break;
-            }
-        } while ((int)(seen - want) < 0);
-        __threadfence();
-    }
-    __syncthreads();
-}
-
-// Block sums of N per-thread values, of which the first `warps` warps hold
-// non-zero ones, into this block's entries of a slot: through shared memory
-// and one warp per value.  FP64 operations are few (two lanes per SM clock)
-// and slow one after the other, so only warps with something to add count.
-template <int N>
-__device__ __forceinline__ void block_partials(Shared& s, const double (&v)[N], int warps,
-                                               double* red, int slot) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp < warps) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) s.lane[i][threadIdx.x] = v[i];
-    }
-    __syncthreads();
-    if (warp < N) {
-        double t[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int w = 0; w < warps; w += 4) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (w + i < warps) t[i] += s.lane[warp][(w + i) * 32 + lane];
-        }
-        const double a = warp_sum((t[0] + t[1]) + (t[2] + t[3]));
-        if (lane == 0) red[((long long)slot * 4 + warp) * gridDim.x + blockIdx.x] = a;
-    }
-}
-
-// After the barrier, one warp: the sum of entry i of a slot over the blocks,
-// in a fixed order (every lane holds it).
-template <int N>
-__device__ __forceinline__ void reduce_slot(const double* red, int slot, double (&out)[N]) {
-    const int lane = threadIdx.x & 31;
-    const double* p = red + (long long)slot * 4 * gridDim.x;
-#pragma unroll
-    for (int i = 0; i < N; ++i) out[i] = 0.0;
-    for (unsigned b = lane; b < gridDim.x; b += 32)
-#pragma unroll
-        for (int i = 0; i < N; ++i) out[i] += __ldcg(p + (long long)i * gridDim.x + b);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int i = 0; i < N; ++i) out[i] += __shfl_xor_sync(0xffffffffu, out[i], o);
-}
-
-// sqrt of each of N values, side by side in the lanes of a warp
-template <int N>
-__device__ __forceinline__ void warp_sqrt(double (&v)[N]) {
-    const int lane = threadIdx.x & 31;
-    double mine = v[0];
-#pragma unroll
-    for (int i = 1; i < N; ++i) mine = lane == i ? v[i] : mine;
-    mine = sqrt(mine);
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = __shfl_sync(0xffffffffu, mine, i);
-}
 
 // ---- the rings through which a warp reads the basis ----
 //
