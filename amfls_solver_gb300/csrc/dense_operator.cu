@@ -586,16 +586,16 @@ bool DenseOperator::product1(bool transpose, const double* x, const Epilogue& ep
     // contiguous (apply = dot of rows); column-major columns are (transpose =
     // dot of columns).
     //
-    // Without the sliced sums: the width controller weighs the measured cost of
-    // this product against the local algebra, and the policies trained on its
-    // decisions earn their gain where it widens.  With the sliced sums (131 -> 27 us,
-    // 16384 x 512 transposed) it never widens on the dense study family, and a
-    // policy has nothing left to gain there.
+    // A level's product goes without the sliced sums: the width controller weighs
+    // its measured cost against the local algebra, and the policies trained on
+    // the controller's decisions earn their gain where it widens.  With the sliced
+    // sums (131 -> 27 us, 16384 x 512 transposed) it never widens on the dense
+    // study family, and a policy has nothing left to gain there.
     const int out_n = transpose ? cols_ : rows_;
     const int in_n = transpose ? rows_ : cols_;
     const long long ld = column_major_ ? rows_ : cols_;
     launch_block<1>(column_major_ == transpose, a_, ld, out_n, in_n, x, in_n, partials_, tmp_,
-                    out_n, s, ep.guard, false);
+                    out_n, s, ep.guard, !ep.level);
     run_epilogue(tmp_, out_n, ep, ep.partials ? ep.partials : scratch_,
                  ep.counter ? ep.counter : counter_ + 1, s);
     return true;

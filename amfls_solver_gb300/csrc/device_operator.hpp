@@ -62,6 +62,7 @@ struct Epilogue {
     const double* dot_vec = nullptr;
     RedResult* red = nullptr;
     const int* guard = nullptr;  // skip the launch's work when *guard == 0
+    bool level = false;  // a width-one level's product: its time feeds the width gate
     // Scratch for the cross-block reduction (one slot of 6 doubles per block
     // and a ticket counter that must start at zero).  When null the operator
     // uses its own, which serialises fused products on one operator.

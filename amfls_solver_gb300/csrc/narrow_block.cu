@@ -13,8 +13,8 @@
 // the rank cutoff (its smallest singular value is at least 1 / ||R^{-1}||_F),
 // ill conditioned or not finite, the host goes on from the projected residual
 // with the rank-revealing path.  A solve of 128 such levels and its checkpoints
-// went from 331 to 59 ms, one of 4 columns on a dense 16384 x 512 matrix from 302
-// to 100 ms (most of it now products and validation).
+// went from 331 to 49 ms, one of 4 columns on a dense 16384 x 512 matrix from 302
+// to 50 ms.
 //
 // FP64 operations bound the projections (one multiply-add per basis element and
 // column at two lanes per SM clock); the kernels carry exactly the columns
@@ -32,6 +32,8 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kTileRows = 64;
+constexpr int kNnThreads = 128;
+constexpr int kApplyThreads = 128;
 
 template <typename F>
 void with_padded(int c, F&& f) {
@@ -133,12 +135,14 @@ panel_tn_kernel(double* const* panels, int n, int k, const double* B, int c, int
 
 // B -= V C: a warp takes R pairs of rows over all panels, 16 lanes a row; the
 // lanes' sums are added by a butterfly that halves the columns a lane holds.
+// Four warps a block, one for each SM quarter: with eight, 1200 rows kept half of
+// the SMs busy (25 -> 20 us at 480 columns and 8 block columns).
 template <int C, int R>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kNnThreads)
 panel_nn_kernel(double* const* panels, int n, int p0, int p1, const double* __restrict__ coeff,
                 int c, double* B) {
     const int lane = threadIdx.x & 31, half = lane >> 4, q = lane & 15;
-    const int warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    const int warp = blockIdx.x * (kNnThreads / 32) + (threadIdx.x >> 5);
     const int first = warp * 2 * R;
     if (first >= n) return;
     double acc[R][C];
@@ -146,7 +150,8 @@ panel_nn_kernel(double* const* panels, int n, int p0, int p1, const double* __re
     for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int j = 0; j < C; ++j) acc[r][j] = 0.0;
-#pragma unroll 2
+    // several panels' loads in flight: a quarter has one warp to hide them
+#pragma unroll(C* R <= 8 ? 4 : 2)
     for (int p = p0; p < p1; ++p) {
         const double2* vp = reinterpret_cast<const double2*>(panels[p]);
         double2 v[R];
@@ -216,9 +221,10 @@ __device__ bool warp_cholesky(double (*G)[kNarrowMax + 1], double (*R)[kNarrowMa
         const double d = G[j][j];
         const bool good = d > 0.0 && isfinite(d);
         ok = ok && good;
-        const double r = good ? sqrt(d) : 1.0, inv = 1.0 / r;
+        const double inv = good ? rsqrt(d) : 1.0;
         if (lane == 0) pivot_inv[j] = inv;
-        if (lane < c) R[j][lane] = lane < j ? 0.0 : lane == j ? r : G[j][lane] * inv;
+        // lane j: the pivot's root (d / sqrt(d))
+        if (lane < c) R[j][lane] = lane < j ? 0.0 : good ? G[j][lane] * inv : lane == j ? 1.0 : G[j][lane];
         __syncwarp();
         for (int t = lane; t < c * c; t += 32) {
             const int i = t / c, l = t % c;
@@ -336,9 +342,9 @@ gram_kernel(const double* X, const double* Y, long long m, int a, int b, int end
                 f->resid2 = trace;
                 // smallest singular value >= 1 / ||R^{-1}||_F, condition <=
                 // ||R||_F ||R^{-1}||_F
-                const double cutoff = cutoff_unit * sqrt(f->scale2);
+                const double unit = 1.01 * cutoff_unit;
                 ok = ok && isfinite(trace) && isfinite(fi) && isfinite(f->scale2) &&
-                     !f->nonfinite && fr * fi < 1e12 && 1.0 > 1.01 * cutoff * sqrt(fi);
+                     !f->nonfinite && fr * fi < 1e12 && 1.0 > unit * unit * f->scale2 * fi;
                 f->ok = ok ? 1 : 0;
             } else {
                 f->ok = f->ok && ok && isfinite(fi) ? 1 : 0;
@@ -357,33 +363,39 @@ void gram_launch(const double* X, const double* Y, long long m, int a, int b, in
     AMFLS_LAUNCHED();
 }
 
-template <int B>
-__global__ void __launch_bounds__(kThreads)
+// A thread takes one row and J of the b columns (blockIdx.y chooses them):
+// with all of them in one thread, 5000 rows of 8 columns gave 20 blocks of 512 FP64
+// operations a thread (12.6 -> 5.9 us).
+template <int J>
+__global__ void __launch_bounds__(kApplyThreads)
 apply_kernel(const double* X, const double* C, int transposed, int ldc, long long m, int a, int b,
              double* Y, double alpha, double beta) {
-    __shared__ double cs[kNarrowMax][B];
-    for (int t = threadIdx.x; t < a * B; t += kThreads) {
-        const int i = t / B, j = t % B;
-        cs[i][j] = j < b ? (transposed ? C[j + i * ldc] : C[i + j * ldc]) : 0.0;
+    __shared__ double cs[kNarrowMax][J];
+    const int j0 = blockIdx.y * J;
+    for (int t = threadIdx.x; t < a * J; t += kApplyThreads) {
+        const int i = t / J, j = j0 + t % J;
+        cs[i][t % J] = j < b ? (transposed ? C[j + i * ldc] : C[i + j * ldc]) : 0.0;
     }
     __syncthreads();
-    for (long long r = blockIdx.x * (long long)kThreads + threadIdx.x; r < m;
-         r += (long long)gridDim.x * kThreads) {
-        double acc[B];
+    for (long long r = blockIdx.x * (long long)kApplyThreads + threadIdx.x; r < m;
+         r += (long long)gridDim.x * kApplyThreads) {
+        double old[J], acc[J];
 #pragma unroll
-        for (int j = 0; j < B; ++j) acc[j] = 0.0;
+        for (int j = 0; j < J; ++j) {
+            old[j] = beta != 0.0 && j0 + j < b ? Y[r + (long long)(j0 + j) * m] : 0.0;
+            acc[j] = 0.0;
+        }
 #pragma unroll 4
         for (int i = 0; i < a; ++i) {
             const double x = X[r + (long long)i * m];
 #pragma unroll
-            for (int j = 0; j < B; ++j) acc[j] = fma(x, cs[i][j], acc[j]);
+            for (int j = 0; j < J; ++j) acc[j] = fma(x, cs[i][j], acc[j]);
         }
 #pragma unroll
-        for (int j = 0; j < B; ++j) {
-            if (j < b) {
-                double* y = Y + r + (long long)j * m;
-                *y = beta == 0.0 ? alpha * acc[j] : fma(alpha, acc[j], beta * *y);
-            }
+        for (int j = 0; j < J; ++j) {
+            if (j0 + j < b)
+                Y[r + (long long)(j0 + j) * m] =
+                    beta == 0.0 ? alpha * acc[j] : fma(alpha, acc[j], beta * old[j]);
         }
     }
 }
@@ -448,11 +460,11 @@ void panel_nn(double* const* panels, long long n, int p0, int p1, const double* 
         constexpr int W = w(), R = W <= 8 ? 4 : 2;
         if (many) {
             const long long warps = (n + 2 * R - 1) / (2 * R);
-            panel_nn_kernel<W, R><<<(unsigned)((warps + 7) / 8), kThreads, 0, s>>>(
+            panel_nn_kernel<W, R><<<(unsigned)((warps + 3) / 4), kNnThreads, 0, s>>>(
                 panels, (int)n, p0, p1, C, c, B);
         } else {
             const long long warps = (n + 1) / 2;
-            panel_nn_kernel<W, 1><<<(unsigned)((warps + 7) / 8), kThreads, 0, s>>>(
+            panel_nn_kernel<W, 1><<<(unsigned)((warps + 3) / 4), kNnThreads, 0, s>>>(
                 panels, (int)n, p0, p1, C, c, B);
         }
     });
@@ -477,10 +489,14 @@ void gram(const double* X, const double* Y, long long m, int a, int b, double* C
 
 void apply(const double* X, const double* C, bool transposed, int ldc, long long m, int a, int b,
            double* Y, double alpha, double beta, cudaStream_t s) {
-    with_padded(b, [&](auto B) {
-        apply_kernel<B()><<<grid_1d(m), kThreads, 0, s>>>(X, C, transposed ? 1 : 0, ldc, m, a, b, Y,
-                                                         alpha, beta);
-    });
+    // one column a thread while that does not give every SM quarter several
+    // warps; beyond, four share the loads of X
+    const int J = m * b <= 32LL * 32 * sm_count() || b < 4 ? 1 : 4;
+    const long long rows = (m + kApplyThreads - 1) / kApplyThreads;
+    const dim3 grid((unsigned)std::max<long long>(1, std::min<long long>(rows, 4LL * grid_cap())),
+                    (unsigned)((b + J - 1) / J));
+    (J == 1 ? apply_kernel<1> : apply_kernel<4>)<<<grid, kApplyThreads, 0, s>>>(
+        X, C, transposed ? 1 : 0, ldc, m, a, b, Y, alpha, beta);
     AMFLS_LAUNCHED();
 }
 

@@ -1492,6 +1492,7 @@ void Workspace::enqueue_level_kernels(cudaStream_t s, int pcap) {
     ep.coef = &dstate_->coupling_eff;
     ep.red = &red_[0];
     ep.guard = &dstate_->go;
+    ep.level = true;
     ep.partials = partials_;
     ep.counter = counter_ + 2;
     if (!op_.product1(true, U_, ep, s)) throw std::runtime_error("operator has no fused device product");
@@ -1582,6 +1583,7 @@ void Workspace::enqueue_level_kernels(cudaStream_t s, int pcap) {
     el.dot_vec = U_;
     el.red = &red_[1];
     el.guard = &dstate_->go;
+    el.level = true;
     el.partials = partials_;
     el.counter = counter_ + 2;
     op_.product1(false, vnew_, el, s);
