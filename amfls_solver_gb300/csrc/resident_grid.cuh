@@ -69,20 +69,43 @@ __device__ __forceinline__ void block_partials(Sh& s, const double (&v)[N], int 
 }
 
 // After the barrier, one warp: the sum of entry i of a slot over the blocks,
-// in a fixed order (every lane holds it).
+// in a fixed order (every lane holds it).  Several values share the additions
+// of one butterfly that halves the values a lane holds (three: six dependent
+// FP64 additions over the lanes instead of fifteen).
 template <int N>
 __device__ __forceinline__ void reduce_slot(const double* red, int slot, double (&out)[N]) {
+    constexpr int M = N <= 1 ? 1 : N <= 2 ? 2 : 4;
     const int lane = threadIdx.x & 31;
     const double* p = red + (long long)slot * 4 * gridDim.x;
+    double v[M];
 #pragma unroll
-    for (int i = 0; i < N; ++i) out[i] = 0.0;
+    for (int i = 0; i < M; ++i) v[i] = 0.0;
     for (unsigned b = lane; b < gridDim.x; b += 32)
 #pragma unroll
-        for (int i = 0; i < N; ++i) out[i] += __ldcg(p + (long long)i * gridDim.x + b);
+        for (int i = 0; i < N; ++i) v[i] += __ldcg(p + (long long)i * gridDim.x + b);
+    int have = M;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = 16; o > 0; o >>= 1) {
+        if (have > 1) {
+            const bool upper = (lane & o) != 0;
+            have >>= 1;
 #pragma unroll
-        for (int i = 0; i < N; ++i) out[i] += __shfl_xor_sync(0xffffffffu, out[i], o);
+            for (int j = 0; j < M / 2; ++j) {
+                if (j < have) {
+                    const double keep = upper ? v[j + have] : v[j];
+                    const double send = upper ? v[j] : v[j + have];
+                    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    // value i ended in the lanes whose top bits spell i
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        out[i] = M == 1 ? v[0]
+                        : __shfl_sync(0xffffffffu, v[0], M == 2 ? i * 16 : (i >> 1) * 16 + (i & 1) * 8);
 }
 
 // sqrt of each of N values, side by side in the lanes of a warp

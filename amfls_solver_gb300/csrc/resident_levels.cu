@@ -136,13 +136,17 @@ __device__ __forceinline__ const unsigned char* take_slot(Shared& s, Ring& k) {
 // ---- V^T r in 4 KB units of the panels, equal shares per block ----
 
 // Shares for a basis of k columns: block b of the first `used` (all of them
-// unless there are fewer units) takes units [total b / used, total (b+1) / used).
+// unless there are fewer than four units for each) takes units
+// [total b / used, total (b+1) / used).  Four units are one for each SM quarter,
+// so more blocks would not finish sooner, and every block adds the segments of
+// all (2000 x 500, V^T r to the norm test: 20.7 -> 16.5 us per level with the
+// shared butterflies of reduce_slot).
 __device__ __forceinline__ void set_shares(Shared& s, int n, int k, int unit_rows) {
     const int P = (k + 31) >> 5;
     const int upp = (n + unit_rows - 1) / unit_rows;
     if (P == s.P && upp == s.upp) return;  // uniform: they change only between block barriers
     const long long total = (long long)P * upp;
-    const int used = (int)min(total, (long long)gridDim.x);
+    const int used = (int)min((total + 3) / 4, (long long)gridDim.x);
     __syncthreads();
     for (int p = threadIdx.x; p < P; p += kT) {
         // the block of unit u: the largest b with total b / used <= u
@@ -264,8 +268,10 @@ __device__ __forceinline__ void sweep_vt(Shared& s, const ResidentArgs& a, Ring&
         const int p = pb + warp;
         if (warp < kSegs && (long long)p * s.upp < ue) {
             double x[4] = {0.0, 0.0, 0.0, 0.0};
+            const int warps = (int)min((long long)kW, s.u1 - s.u0);  // the others' are zero
+            for (int w = 0; w < warps; w += 4)
 #pragma unroll
-            for (int w = 0; w < kW; ++w) x[w & 3] += s.seg[warp][w][lane];
+                for (int i = 0; i < 4; ++i) x[i] += s.seg[warp][w + i][lane];
             a.part[((long long)blockIdx.x + p) * 32 + lane] = (x[0] + x[1]) + (x[2] + x[3]);
         }
         if ((long long)(pb + kSegs) * s.upp < s.u1) __syncthreads();  // seg is reused
@@ -281,7 +287,7 @@ __device__ __forceinline__ void gather_coefficients(Shared& s, const ResidentArg
         const int p = j >> 5;
         const int b1 = s.seg_last[p];
         const double* src = a.part + (long long)p * 32 + (j & 31);
-        double t = 0.0;
+        double x[4] = {0.0, 0.0, 0.0, 0.0};
         for (int b = s.seg_first[p]; b <= b1; b += 8) {
             double v[8];
 #pragma unroll
@@ -289,8 +295,9 @@ __device__ __forceinline__ void gather_coefficients(Shared& s, const ResidentArg
                 v[i] = b + i <= b1 ? __ldcg(src + (long long)(b + i) * 32) : 0.0;
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                if (b + i <= b1) t += v[i];
+                if (b + i <= b1) x[i & 3] += v[i];
         }
+        double t = (x[0] + x[1]) + (x[2] + x[3]);
         t *= scale;
         if (j >= k) t = 0.0;
         c[j] = t;
@@ -702,8 +709,11 @@ __global__ void __launch_bounds__(kT, 1) resident_levels_kernel(ResidentArgs a) 
                             double q2 = 0.0;
                             for (int j = lane; j < k; j += 32) q2 = fma(coeff[j], coeff[j], q2);
                             q2 = warp_sum(q2);
+                            warp_sqrt(nb);
                             if (lane == 0) {
-                                const double before = sqrt(nb[1]);
+                                const double before = nb[1];
+                                s.st.right_scale = nb[0];
+                                s.st.norm_before = before;
                                 const double bound = kReducedCoeffBound * before;
                                 const bool redo =
                                     !(isfinite(q2) && isfinite(before)) || q2 > bound * bound;
@@ -750,6 +760,16 @@ __global__ void __launch_bounds__(kT, 1) resident_levels_kernel(ResidentArgs a) 
                         failed = true;
                         break;
                     }
+                    if (pass == 1 && warp == kW - 1) {
+                        // a warp with few coefficients: off the decision's path
+                        double nb[2];
+                        reduce_slot(a.red, kRedRight, nb);
+                        warp_sqrt(nb);
+                        if (lane == 0) {
+                            s.st.right_scale = nb[0];
+                            s.st.norm_before = nb[1];
+                        }
+                    }
                     gather_coefficients(s, a, k, coeff, 1.0);
                     part = sweep_vc(s, a, ring, r0, r1, coeff, piece);
                     sparse_partial<16>(s, part, a.red, pass == 1 ? kRedNorm : kRedNorm2);
@@ -764,18 +784,22 @@ __global__ void __launch_bounds__(kT, 1) resident_levels_kernel(ResidentArgs a) 
                 }
             }
             if (warp == 0) {
-                double nb[2], after[1] = {0.0};
-                reduce_slot(a.red, kRedRight, nb);
-                if (k > 0) reduce_slot(a.red, pass == 1 ? kRedNorm : kRedNorm2, after);
-                double v[3] = {nb[0], nb[1], k > 0 ? after[0] : nb[1]};
-                warp_sqrt(v);
+                double v[2] = {0.0, 0.0};
+                if (k > 0) {
+                    double after[1];
+                    reduce_slot(a.red, pass == 1 ? kRedNorm : kRedNorm2, after);
+                    v[1] = sqrt(after[0]);
+                } else {
+                    reduce_slot(a.red, kRedRight, v);
+                    warp_sqrt(v);
+                }
                 if (lane == 0) {
-                    if (pass < 2) {
+                    if (k == 0) {
                         s.st.right_scale = v[0];
                         s.st.norm_before = v[1];
                     }
-                    s.st.norm_after = v[2];
-                    s.st.second_pass = k > 0 && pass < 2 && dgks_again(v[1], v[2]) ? 1 : 0;
+                    s.st.norm_after = v[1];
+                    s.st.second_pass = k > 0 && pass < 2 && dgks_again(s.st.norm_before, v[1]) ? 1 : 0;
                     if (!s.st.second_pass) decide_right(&s.st, a.ml, n);
                     if (writer) s.st.t_mark = global_ns();
                 }
