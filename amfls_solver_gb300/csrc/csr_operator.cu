@@ -26,6 +26,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
+#include <cstring>
 #include <memory>
 #include <numeric>
 #include <stdexcept>
@@ -75,6 +76,21 @@ __global__ void check_offsets_kernel(const long long* off, int rows, long long n
         }
         bins[r] = bin;
     }
+}
+
+// row numbers, and how many rows each bin has
+constexpr int kLengthBins = 6;
+__global__ void bin_rows_kernel(const int* bins, int rows, int* ids, int* counts) {
+    __shared__ int local[kLengthBins];
+    if (threadIdx.x < kLengthBins) local[threadIdx.x] = 0;
+    __syncthreads();
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
+        atomicAdd(&local[bins[r]], 1);
+        ids[r] = r;
+    }
+    __syncthreads();
+    if (threadIdx.x < kLengthBins && local[threadIdx.x])
+        atomicAdd(&counts[threadIdx.x], local[threadIdx.x]);
 }
 
 __global__ void expand_rows_kernel(const long long* off, const long long* idx64,
@@ -271,12 +287,7 @@ struct TileStore {
         return t;
     }
     void release() {
-        cudaFree(tiles);
-        cudaFree(split);
-        cudaFree(chain);
-        cudaFree(long_rows);
-        cudaFree(long_count);
-        cudaFree(long_part);
+        cudaFree(tiles);  // the one allocation
         *this = TileStore{};
     }
 };
@@ -433,26 +444,31 @@ void make_tiles(const std::vector<long long>& off, int count, int E, int C, bool
     ts.chains = chains;
     const size_t nt = std::max<size_t>(1, tiles.size()), nl = std::max<size_t>(1, long_rows.size());
     const size_t nc = std::max<size_t>(1, chain.size());
-    AMFLS_CUDA(cudaMalloc(&ts.tiles, sizeof(int4) * nt));
-    AMFLS_CUDA(cudaMalloc(&ts.split, sizeof(int) * nt));
-    AMFLS_CUDA(cudaMalloc(&ts.chain, sizeof(int2) * nc));
-    AMFLS_CUDA(cudaMalloc(&ts.long_rows, sizeof(int2) * nl));
-    AMFLS_CUDA(cudaMalloc(&ts.long_count, sizeof(unsigned) * nl));
-    AMFLS_CUDA(cudaMalloc(&ts.long_part, sizeof(double) * C * nt));
-    AMFLS_CUDA(cudaMemsetAsync(ts.long_count, 0, sizeof(unsigned) * nl, stream));
-    if (!tiles.empty()) {
+    // one allocation: tiles | long_part | chain | long_rows | split | long_count,
+    // and one copy of the tables through a host image of it
+    const size_t at_part = sizeof(int4) * nt, at_chain = at_part + sizeof(double) * C * nt;
+    const size_t at_long = at_chain + sizeof(int2) * nc, at_split = at_long + sizeof(int2) * nl;
+    const size_t at_count = at_split + sizeof(int) * nt, bytes = at_count + sizeof(unsigned) * nl;
+    unsigned char* base = nullptr;
+    AMFLS_CUDA(cudaMalloc(&base, bytes));
+    ts.tiles = reinterpret_cast<int4*>(base);
+    ts.long_part = reinterpret_cast<double*>(base + at_part);
+    ts.chain = reinterpret_cast<int2*>(base + at_chain);
+    ts.long_rows = reinterpret_cast<int2*>(base + at_long);
+    ts.split = reinterpret_cast<int*>(base + at_split);
+    ts.long_count = reinterpret_cast<unsigned*>(base + at_count);
+    std::vector<unsigned char> image(bytes - at_chain, 0);
+    auto lay = [&](const auto& v, size_t at) {
+        if (!v.empty()) std::memcpy(image.data() + at - at_chain, v.data(), sizeof(v[0]) * v.size());
+    };
+    lay(chain, at_chain);
+    lay(long_rows, at_long);
+    lay(split, at_split);
+    if (!tiles.empty())
         AMFLS_CUDA(cudaMemcpyAsync(ts.tiles, tiles.data(), sizeof(int4) * tiles.size(),
                                    cudaMemcpyHostToDevice, stream));
-        AMFLS_CUDA(cudaMemcpyAsync(ts.split, split.data(), sizeof(int) * split.size(),
-                                   cudaMemcpyHostToDevice, stream));
-    }
-    if (!chain.empty())
-        AMFLS_CUDA(cudaMemcpyAsync(ts.chain, chain.data(), sizeof(int2) * chain.size(),
-                                   cudaMemcpyHostToDevice, stream));
-    if (!long_rows.empty())
-        AMFLS_CUDA(cudaMemcpyAsync(ts.long_rows, long_rows.data(),
-                                   sizeof(int2) * long_rows.size(), cudaMemcpyHostToDevice,
-                                   stream));
+    AMFLS_CUDA(cudaMemcpyAsync(base + at_chain, image.data(), image.size(), cudaMemcpyHostToDevice,
+                               stream));
     AMFLS_CUDA(cudaStreamSynchronize(stream));  // host vectors go out of scope
 }
 
@@ -725,41 +741,43 @@ void CsrOperator::release() {
 void CsrOperator::build_bins(Side& s, const int* d_bins, cudaStream_t stream) {
     // stable sort rows by bin -> perm; bin boundaries from a histogram
     const int n = s.count;
-    int *keys_in = nullptr, *keys_out = nullptr, *vals_in = nullptr;
-    AMFLS_CUDA(cudaMallocAsync(&keys_out, sizeof(int) * std::max(1, n), stream));
-    AMFLS_CUDA(cudaMallocAsync(&vals_in, sizeof(int) * std::max(1, n), stream));
+    int *keys_out = nullptr, *vals_in = nullptr, *counts = nullptr;
+    void* tmp = nullptr;
     AMFLS_CUDA(cudaMalloc(&s.perm, sizeof(int) * std::max(1, n)));
-    keys_in = const_cast<int*>(d_bins);
-    {
-        std::vector<int> seq(n);
-        for (int i = 0; i < n; ++i) seq[i] = i;
-        AMFLS_CUDA(cudaMemcpyAsync(vals_in, seq.data(), sizeof(int) * n, cudaMemcpyHostToDevice,
-                                   stream));
+    auto free_all = [&] {
+        stream_free(keys_out, stream);
+        stream_free(vals_in, stream);
+        stream_free(counts, stream);
+        stream_free(tmp, stream);
+    };
+    try {
+        stream_alloc(&keys_out, sizeof(int) * std::max(1, n), stream);
+        stream_alloc(&vals_in, sizeof(int) * std::max(1, n), stream);
+        stream_alloc(&counts, sizeof(int) * kLengthBins, stream);
+        AMFLS_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * kLengthBins, stream));
+        bin_rows_kernel<<<setup_grid(n), 256, 0, stream>>>(d_bins, n, vals_in, counts);
+        AMFLS_LAUNCHED();
         size_t tmp_bytes = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys_in, keys_out, vals_in, s.perm, n,
-                                        0, 3, stream);
-        void* tmp = nullptr;
-        AMFLS_CUDA(cudaMallocAsync(&tmp, std::max<size_t>(tmp_bytes, 1), stream));
-        AMFLS_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys_in, keys_out, vals_in,
+        AMFLS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, d_bins, keys_out, vals_in,
                                                    s.perm, n, 0, 3, stream));
-        std::vector<int> sorted(n);
-        AMFLS_CUDA(cudaMemcpyAsync(sorted.data(), keys_out, sizeof(int) * n,
-                                   cudaMemcpyDeviceToHost, stream));
-        AMFLS_CUDA(cudaStreamSynchronize(stream));
-        AMFLS_CUDA(cudaFreeAsync(tmp, stream));
-        long long counts[6] = {0, 0, 0, 0, 0, 0};
-        for (int v : sorted) counts[v]++;
+        AMFLS_CUDA(cudaMallocAsync(&tmp, std::max<size_t>(tmp_bytes, 1), stream));
+        AMFLS_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, d_bins, keys_out, vals_in,
+                                                   s.perm, n, 0, 3, stream));
+        int host[kLengthBins] = {};
+        read_back(host, counts, stream, kLengthBins);
         s.bins.warp_start[0] = 0;
         s.bins.row_start[0] = 0;
-        for (int b = 0; b < 6; ++b) {
+        for (int b = 0; b < kLengthBins; ++b) {
             const long long rows_per_warp = 32 >> b;
             s.bins.warp_start[b + 1] =
-                s.bins.warp_start[b] + (counts[b] + rows_per_warp - 1) / rows_per_warp;
-            s.bins.row_start[b + 1] = s.bins.row_start[b] + (int)counts[b];
+                s.bins.warp_start[b] + (host[b] + rows_per_warp - 1) / rows_per_warp;
+            s.bins.row_start[b + 1] = s.bins.row_start[b] + host[b];
         }
+    } catch (...) {
+        free_all();
+        throw;
     }
-    AMFLS_CUDA(cudaFreeAsync(keys_out, stream));
-    AMFLS_CUDA(cudaFreeAsync(vals_in, stream));
+    free_all();
 }
 
 void CsrOperator::build(const long long* d_off, const long long* d_idx, const double* d_val,

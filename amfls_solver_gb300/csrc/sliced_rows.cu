@@ -78,10 +78,7 @@ int grid_for(long long items) {
 }  // namespace
 
 void Store::release() {
-    cudaFree(tasks);
-    cudaFree(lanes);
-    cudaFree(idx);
-    cudaFree(val);
+    cudaFree(val);  // the one allocation
     *this = Store{};
 }
 
@@ -133,10 +130,14 @@ void build(Store& store, const long long* off, const int* idx, const double* val
                                    stream));
         AMFLS_CUDA(cudaStreamSynchronize(stream));
         const size_t entries = 32 * (size_t)std::max(1, total);
-        AMFLS_CUDA(cudaMalloc(&store.tasks, sizeof(int2) * std::max(1, ntasks)));
-        AMFLS_CUDA(cudaMalloc(&store.lanes, sizeof(int2) * 32 * (size_t)std::max(1, ntasks)));
-        AMFLS_CUDA(cudaMalloc(&store.idx, sizeof(int) * entries));
-        AMFLS_CUDA(cudaMalloc(&store.val, sizeof(double) * entries));
+        // one allocation: val, lanes, idx and tasks are whole multiples of 128 bytes
+        // but for the last
+        const size_t slots = (size_t)std::max(1, ntasks);
+        AMFLS_CUDA(cudaMalloc(&store.val, (sizeof(double) + sizeof(int)) * entries +
+                                              sizeof(int2) * 33 * slots));
+        store.lanes = reinterpret_cast<int2*>(store.val + entries);
+        store.idx = reinterpret_cast<int*>(store.lanes + 32 * slots);
+        store.tasks = reinterpret_cast<int2*>(store.idx + entries);
         fill_kernel<<<grid_for(32LL * ntasks), 256, 0, stream>>>(
             g, sorted, lens_out, first, ntasks, off, idx, val, store.tasks, store.lanes, store.idx,
             store.val);
