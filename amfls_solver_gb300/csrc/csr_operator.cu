@@ -415,7 +415,9 @@ void make_tiles(const std::vector<long long>& off, int count, int E, int C, bool
             while (r < count && length(r) <= longer_than && off[r + 1] - e0 <= E && r - r0 < E)
                 ++r;
             tiles.push_back(make_int4(r0, r, (int)e0, (int)off[r]));
-            split.push_back(kRowBlock);
+            split.push_back(
+                C == 1 ? kRowBlock
+                       : kRowBlock | split_bits(r - r0, [&](int i) { return length(r0 + i); }));
             cost.push_back(3);
         }
     }

@@ -72,6 +72,8 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kE1 = 256;     // elements per tile, single-column products
 constexpr int kEC = 64;      // elements per tile, 2..8 columns
 constexpr int kSeqMax = 64;  // longest row of a multi-column row block
+// rows of a block that all lanes may sum together (multi-column products)
+constexpr int kSplitRow = 8;
 constexpr int kRowTaskTiles = 16;  // a row of up to 16 E nonzeros is one warp task
 static_assert(kEC <= kSeqMax, "multi-column tiles sum every row sequentially");
 constexpr int kChainMax = 64;     // longest row summed as a per-lane chain (C == 1)
@@ -81,13 +83,49 @@ constexpr int kChainStep = 8;     // elements per row staged at a time
 constexpr int kFlatRows = 256;    // rows of a group whose rows hold at most one nonzero
 // task kinds (Table::split): row block, whole long row, chain group; q >= 0
 // is a slice of long row q
-constexpr int kRowBlock = -1, kWholeRow = -2, kChainGroup = -3;
+constexpr int kRowBlock = -64, kWholeRow = -2, kChainGroup = -3;
+
+// A row block of a multi-column table carries a bit for each of C = 2, 4, 8
+// columns that says whether all 32 / C groups sum its rows of more than
+// kSplitRow nonzeros together (strided, then a butterfly).  A batch of 32 / C rows
+// takes as many FP64 steps as its longest row, and an idle lane's step takes
+// the pipe's time all the same; the bit is set where the split saves a fifth of
+// the block's steps.  Microseconds per product without and with it: 33 nonzeros in
+// every row, so that a block holds one (50000 x 12000), 105 and 60 for 8
+// columns, 100 and 39 for 2; power-law rows (200000 x 50000, 20 on average) 93 and 91
+// for 8, 66 and 60 for 4.
+constexpr int split_bit(int c) { return c == 2 ? 1 : c == 4 ? 2 : 4; }
+constexpr bool is_row_block(int q) { return q <= kRowBlock + 7; }
+
+// The bits of the block of `rows` rows with the given lengths.
+template <typename Length>
+int split_bits(int rows, Length&& length) {
+    int bits = 0;
+    for (int c = 2; c <= 8; c *= 2) {
+        const int groups = 32 / c, log = c == 2 ? 4 : c == 4 ? 3 : 2;
+        long long whole = 0, split = 0;
+        for (int i0 = 0; i0 < rows; i0 += groups) {
+            long long most = 0, rest = 0;
+            for (int i = i0; i < rows && i < i0 + groups; ++i) {
+                const long long len = length(i);
+                most = len > most ? len : most;
+                if (len > kSplitRow) split += (len + groups - 1) / groups + log;
+                else rest = len > rest ? len : rest;
+            }
+            whole += most;
+            split += rest;
+        }
+        if (5 * split <= 4 * whole) bits |= split_bit(c);
+    }
+    return bits;
+}
 
 struct Table {
     // row block, whole row or slice: {first row, end row, first element, end
     // element}; chain group: {first position in chain, rows, longest row, 0}
     const int4* tiles = nullptr;
-    // kRowBlock, kWholeRow, kChainGroup, or q >= 0: a slice of long row q
+    // kRowBlock (with its split bits), kWholeRow, kChainGroup, or q >= 0: a slice
+    // of long row q
     // (rows longer than kRowTaskTiles E)
     const int* split = nullptr;
     // the rows of the chain groups, group by group: {row, first element}, the
@@ -304,7 +342,7 @@ tile_product_kernel(const int* __restrict__ off, const int* __restrict__ idx,
                     if (ncols > 0) y[ce.x] = static_cast<double>(acc);
                 }
             }
-        } else if (q != kRowBlock) {
+        } else if (!is_row_block(q)) {
             // a whole long row (kWholeRow) or a slice of one (q >= 0), through
             // registers: group g = lane / C takes elements g, g + 32 / C, ...,
             // lane c of the group column c
@@ -324,8 +362,11 @@ tile_product_kernel(const int* __restrict__ off, const int* __restrict__ idx,
 #pragma unroll
                 for (int u = 0; u < kStep; ++u)
                     xv[u] = jv[u] >= 0 ? to_acc<A>(__ldg(x + (long long)jv[u] * C + cl)) : A(0);
+                // a step beyond the row's end would take its slot of the FP64
+                // pipe all the same (rows of 80: 20 steps, not 32)
 #pragma unroll
-                for (int u = 0; u < kStep; ++u) part = fma(av[u], xv[u], part);
+                for (int u = 0; u < kStep; ++u)
+                    if (base + kG * u < d.w) part = fma(av[u], xv[u], part);
             }
             for (int o = 16; o >= C; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
             double acc[C];
@@ -416,10 +457,32 @@ tile_product_kernel(const int* __restrict__ off, const int* __restrict__ idx,
                 // C lanes per row (lane c of the group takes column c), 32 / C
                 // rows at a time; rows of these tiles have at most kEC <=
                 // kSeqMax nonzeros
+                // where the table says so, rows of more than kSplitRow are summed
+                // by all groups together first (see split_bits)
                 constexpr int kGroups = 32 / C;
                 const int g = lane / C, c = lane % C;
+                const bool split = (q & split_bit(C)) != 0;
+                if (split) {
+                    for (int i0 = 0; i0 < R; i0 += 32) {
+                        const int len = i0 + lane < R ? ro[i0 + lane + 1] - ro[i0 + lane] : 0;
+                        unsigned m = __ballot_sync(0xffffffffu, len > kSplitRow);
+                        for (; m; m &= m - 1) {
+                            const int i = i0 + __ffs(m) - 1;
+                            const int b0 = ro[i], b1 = ro[i + 1];
+                            A acc = 0;
+                            for (int e = b0 + g; e < b1; e += kGroups)
+                                acc = fma(vs[e], xs[e * C + c], acc);
+#pragma unroll
+                            for (int o = 16; o >= C; o >>= 1)
+                                acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                            if (g == 0 && c < ncols) y[d.x + i + c * ldy] = static_cast<double>(acc);
+                        }
+                    }
+                }
+                const int limit = split ? kSplitRow : E;
                 for (int i = g; i < R; i += kGroups) {
                     const int b0 = ro[i], b1 = ro[i + 1];
+                    if (b1 - b0 > limit) continue;
                     A acc = 0;
                     for (int e = b0; e < b1; ++e) acc = fma(vs[e], xs[e * C + c], acc);
                     if (c < ncols) y[d.x + i + c * ldy] = static_cast<double>(acc);
