@@ -260,7 +260,9 @@ __global__ void __launch_bounds__(kT, 1) resident_baseline_kernel(BaselineArgs a
         if (s.stop) break;
     }
     __syncthreads();
-    if (!s.stop && !s.bad && !s.failed && s.pending) {
+    const bool finish = !s.stop && !s.bad && !s.failed && s.pending;
+    __syncthreads();  // warp 0 may set s.bad from here on
+    if (finish) {
         if (warp == 0) settle_scalars();
         __syncthreads();
         if (!s.bad) commit();
