@@ -125,7 +125,14 @@ panel_tn_kernel(double* const* panels, int n, int k, const double* B, int c, int
     for (int t = threadIdx.x; t < C * 32; t += kThreads) {
         const double* s = partials + (long long)p * chunks * C * 32 + t;
         double x[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int ch = 0; ch < chunks; ++ch) x[ch & 3] += __ldcg(s + (long long)ch * C * 32);
+        for (int ch = 0; ch < chunks; ch += 8) {  // eight loads on their way
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                v[u] = ch + u < chunks ? __ldcg(s + (long long)(ch + u) * C * 32) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) x[u & 3] += v[u];
+        }
         double v = (x[0] + x[1]) + (x[2] + x[3]);
         if (p * 32 + (t & 31) >= k) v = 0.0;
         out[(long long)p * C * 32 + t] = v;
@@ -288,9 +295,16 @@ gram_kernel(const double* X, const double* Y, long long m, int a, int b, int end
     // warp w adds every fourth block, four chains each
     for (int o = lane; o < kOut; o += 32) {
         double x[4] = {0.0, 0.0, 0.0, 0.0};
-        int u = 0;
-        for (int g = warp; g < (int)gridDim.x; g += kWarps, ++u)
-            x[u & 3] += __ldcg(partials + (long long)g * kOut + o);
+        for (int g = warp; g < (int)gridDim.x; g += 4 * kWarps) {
+            double v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                v[u] = g + u * kWarps < (int)gridDim.x
+                           ? __ldcg(partials + (long long)(g + u * kWarps) * kOut + o)
+                           : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] += v[u];
+        }
         red[warp][o] = (x[0] + x[1]) + (x[2] + x[3]);
     }
     __syncthreads();
