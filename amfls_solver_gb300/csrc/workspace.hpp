@@ -133,6 +133,7 @@ private:
     // (the destructor, and a constructor that fails after allocating)
     void release() noexcept;
     void enqueue_level_kernels(cudaStream_t s, int pcap);
+    int resident_interval_grid() const;
     void run_resident(int levels, int target_depth);
     void build_graph(int pcap);
     void invalidate_graph();
