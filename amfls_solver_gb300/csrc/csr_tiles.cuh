@@ -87,7 +87,8 @@ constexpr int kRowBlock = -64, kWholeRow = -2, kChainGroup = -3;
 
 // A row block of a multi-column table carries a bit for each of C = 2, 4, 8
 // columns that says whether all 32 / C groups sum its rows of more than
-// kSplitRow nonzeros together (strided, then a butterfly).  A batch of 32 / C rows
+// kSplitRow nonzeros together (strided, then a butterfly) in FP64 products; FP32
+// sums have no FP64 steps to save and stay one chain a row.  A batch of 32 / C rows
 // takes as many FP64 steps as its longest row, and an idle lane's step takes
 // the pipe's time all the same; the bit is set where the split saves a fifth of
 // the block's steps.  Microseconds per product without and with it: 33 nonzeros in
@@ -458,10 +459,10 @@ tile_product_kernel(const int* __restrict__ off, const int* __restrict__ idx,
                 // rows at a time; rows of these tiles have at most kEC <=
                 // kSeqMax nonzeros
                 // where the table says so, rows of more than kSplitRow are summed
-                // by all groups together first (see split_bits)
+                // in FP64 by all groups together first (see split_bits)
                 constexpr int kGroups = 32 / C;
                 const int g = lane / C, c = lane % C;
-                const bool split = (q & split_bit(C)) != 0;
+                const bool split = std::is_same_v<A, double> && (q & split_bit(C)) != 0;
                 if (split) {
                     for (int i0 = 0; i0 < R; i0 += 32) {
                         const int len = i0 + lane < R ? ro[i0 + lane + 1] - ro[i0 + lane] : 0;
