@@ -728,7 +728,13 @@ __global__ void __launch_bounds__(kT, 1) resident_levels_kernel(ResidentArgs a) 
                         pass = 1;
                         if (!copy) {  // the copy's pieces are not used
                             while (ring.taken < ring.issued) take_slot(s, ring);
-                            __syncthreads();
+                            // the FP64 pass writes its sums to a.part, from which
+                            // other blocks may still be reading the copy's
+                            grid_barrier(s, a.barrier);
+                            if (s.failed) {
+                                failed = true;
+                                break;
+                            }
                         } else {
                             // narrow in place: element j's float lies before its double
                             float* c32 = reinterpret_cast<float*>(coeff);
