@@ -943,17 +943,13 @@ __global__ void __launch_bounds__(kT, 1) resident_levels_kernel(ResidentArgs a) 
 
 template <int kStorage>
 void launch(const ResidentArgs& args, int grid, int k_max, cudaStream_t stream) {
-    const size_t smem = kSharedBytes + kRingBytes + fold_bytes<kStorage>() +
-                        sizeof(double) * 32 * (size_t)((k_max + 31) / 32);
+    const size_t fixed = kSharedBytes + kRingBytes + fold_bytes<kStorage>();
+    const size_t smem = fixed + sizeof(double) * 32 * (size_t)((k_max + 31) / 32);
     auto kernel = resident_levels_kernel<kStorage>;
-    static const bool ready = [] {
-        AMFLS_CUDA(cudaFuncSetAttribute(resident_levels_kernel<kStorage>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(kSharedBytes + kRingBytes + fold_bytes<kStorage>() +
-                                              sizeof(double) * kResidentMaxBasis)));
-        return true;
-    }();
-    (void)ready;
+    // the limit is the current device's: set at every launch, to the same value
+    // by every thread
+    AMFLS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(fixed + sizeof(double) * kResidentMaxBasis)));
     ResidentArgs copy = args;
     void* params[] = {&copy};
     AMFLS_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(grid),
