@@ -274,8 +274,8 @@ public:
     // Takes half-steps from p until `target` are done (true) or one is handed
     // back (false: p is where the general path goes on).  p's indices say which of
     // each pair of vectors is the current one afterwards.
-    bool advance(BaselinePosition& p, int target) {
-        const int from = p.pos;
+    bool advance(BaselinePosition& p, long long target) {
+        const long long from = p.pos;
         p.u = p.v = 0;
         BaselineState st{};
         st.now = p;
@@ -362,7 +362,7 @@ SolveResult solve_lsqr(const DeviceOperator& op, const double* d_b, const Baseli
     double rho = 0.0, cs = 1.0, sn = 0.0;
     int evaluated = 0;  // the last certified iteration
     // half-steps done: A's in 2i, A^T's in 2i + 1
-    for (int pos = 0; pos < 2 * max_it;) {
+    for (long long pos = 0; pos < 2LL * max_it;) {
         bool finite = true, breakdown = false, at_iterate = false;
         if (device.available()) {
             BaselineArgs& g = device.args();
@@ -371,7 +371,7 @@ SolveResult solve_lsqr(const DeviceOperator& op, const double* d_b, const Baseli
             BaselinePosition p{};
             p.alpha = alpha, p.beta = beta, p.rho = rho, p.rhobar = rhobar;
             p.cbar = cs, p.sbar = sn, p.zetabar = phibar, p.pos = pos;
-            at_iterate = device.advance(p, 2 * cand.next((pos + 1) / 2, max_it) - 1);
+            at_iterate = device.advance(p, 2LL * cand.next((int)((pos + 1) / 2), max_it) - 1);
             alpha = p.alpha, beta = p.beta, rho = p.rho, rhobar = p.rhobar;
             cs = p.cbar, sn = p.sbar, phibar = p.zetabar, pos = p.pos;
             if (p.u) std::swap(u, av), std::swap(x, nx);
@@ -405,7 +405,7 @@ SolveResult solve_lsqr(const DeviceOperator& op, const double* d_b, const Baseli
             at_iterate = true;
             ++pos;
         }
-        const int it = (pos + 1) / 2;
+        const int it = (int)((pos + 1) / 2);
         if (at_iterate && (cand.should_evaluate(it) || breakdown || !finite || it == max_it)) {
             cand.evaluate(x, it);
             evaluated = it;
@@ -508,10 +508,10 @@ SolveResult solve_lsmr(const DeviceOperator& op, const double* d_b, const Baseli
             g.w[0] = h, g.w[1] = nh, g.hbar[0] = hbar, g.hbar[1] = nhbar;
             BaselinePosition p{};
             p.alpha = alpha, p.rho = rho, p.rhobar = rhobar, p.cbar = cbar, p.sbar = sbar;
-            p.alphabar = alphabar, p.zetabar = zetabar, p.pos = 2 * it;
-            const bool reached = device.advance(p, 2 * cand.next(it, max_it));
+            p.alphabar = alphabar, p.zetabar = zetabar, p.pos = 2LL * it;
+            const bool reached = device.advance(p, 2LL * cand.next(it, max_it));
             alpha = p.alpha, rho = p.rho, rhobar = p.rhobar, cbar = p.cbar, sbar = p.sbar;
-            alphabar = p.alphabar, zetabar = p.zetabar, it = p.pos / 2;
+            alphabar = p.alphabar, zetabar = p.zetabar, it = (int)(p.pos / 2);
             if (p.u) std::swap(u, av);
             if (p.v) std::swap(v, atu), std::swap(x, nx), std::swap(h, nh), std::swap(hbar, nhbar);
             if (reached) {

@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kT, 1) resident_baseline_kernel(BaselineArgs a
         s.mark = global_ns();
     }
     __syncthreads();
-    const int target = a.st->target;
+    const long long target = a.st->target;
     // the rotations of the pending half-step (warp 0)
     auto settle_scalars = [&] {
         BaselinePosition p = s.now;

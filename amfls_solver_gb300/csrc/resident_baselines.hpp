@@ -13,14 +13,14 @@ namespace amfls_gpu {
 // its rotation in cbar and sbar, phibar in zetabar.
 struct BaselinePosition {
     double alpha, beta, rho, rhobar, cbar, sbar, alphabar, zetabar;
-    int pos;
+    long long pos;  // twice the iterations: past int for the largest limits
     int u, v;  // u's buffer; v's (and LSQR's w, LSMR's x, h, hbar); LSQR's x goes with u
 };
 
 struct BaselineState {
     BaselinePosition now;   // where the kernel stopped
     BaselinePosition back;  // the last unit's start, for a vector that was not finite
-    int target;             // half-steps to stop after
+    long long target;       // half-steps to stop after
     int handed_back;        // `now` is a step that the general path has to take
     int nonfinite[2];       // a vector was not finite, of half-steps in turn
     int timeout;
