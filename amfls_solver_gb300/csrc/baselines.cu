@@ -248,13 +248,15 @@ private:
 };
 
 // The resident iterations of one solve; unavailable without the operator's
-// tables.
+// tables or with a row or column that is far longer than the others.
 class Resident {
 public:
     Resident(const DeviceOperator& op, Run& run, bool lsmr, double damp)
         : run_(run), lsmr_(lsmr) {
         ResidentOperator view;
-        if (!op.resident(&view) || view.augmented) return;
+        if (!op.resident(&view) || view.augmented ||
+            resident_excess(view) > kResidentIterationExcess)
+            return;
         grid_ = sm_count();
         args_.a = view.a;
         args_.t = view.t;

@@ -68,7 +68,7 @@ std::vector<int> sm_shares(const std::vector<BatchItem>& items, const std::vecto
     for (int p = 0; p < count; ++p) {
         ResidentOperator view;
         const DeviceOperator& op = *items[order[p]].op;
-        if (op.resident(&view)) weight[p] = std::sqrt(cost_estimate(op));
+        if (resident_levels(op, &view)) weight[p] = std::sqrt(cost_estimate(op));
     }
     std::vector<int> share(count, 0);
     for (int p = 0; p < count; ++p) {
@@ -107,7 +107,7 @@ std::vector<BatchOutcome> solve_amfls_batch(const std::vector<BatchItem>& items,
     workers = std::min(workers, count);
     const bool resident = std::all_of(items.begin(), items.end(), [](const BatchItem& it) {
         ResidentOperator view;
-        return it.op->resident(&view);
+        return resident_levels(*it.op, &view);
     });
     if (resident) workers = std::min(workers, kResidentStreams);
     std::vector<int> order(count);

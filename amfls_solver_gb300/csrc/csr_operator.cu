@@ -1112,6 +1112,8 @@ bool CsrOperator::resident(ResidentOperator* view) const {
     view->rows = rows_;
     view->cols = cols_;
     view->nonzeros = nnz_;
+    view->longest_row = max_row_nnz_;
+    view->longest_col = max_col_nnz_;
     return true;
 }
 

@@ -1315,7 +1315,7 @@ Workspace::Workspace(const DeviceOperator& op, const double* d_b, double regular
             AMFLS_CUDA(cudaMemsetAsync(red_tickets_, 0, sizeof(unsigned) * (max_panels + 1),
                                        stream_));
         }
-        if (resident_sms > 0 && op_.resident(&resident_op_)) {
+        if (resident_sms > 0 && resident_levels(op_, &resident_op_)) {
             resident_grid_ = std::min(resident_sms, sm_count());
             // sized for the largest grid of an interval
             stream_alloc(&resident_red_, sizeof(double) * resident_red_doubles(sm_count()),
