@@ -16,10 +16,11 @@
 // (graphs of different streams ran one at a time: 48 problems, 16 workers,
 // 12.5 s against 7.9 s).
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cmath>
+#include <cstdlib>
 #include <exception>
+#include <mutex>
 #include <numeric>
 #include <stdexcept>
 #include <string>
@@ -36,11 +37,16 @@ namespace amfls_gpu {
 namespace {
 
 constexpr int kMinShare = 4;
-// Streams of resident solves that run side by side: the driver maps streams to
-// eight hardware queues (its default), and kernels behind a resident one in
-// the same queue wait for it.  1500-column problems on 8 SMs each: 8 in 50 ms, 9
-// in 75 ms, 16 in 171 ms; two rounds of eight on 17 SMs take 68 ms.
-constexpr int kResidentStreams = 8;
+// Resident solves that run side by side: the driver maps streams to
+// CUDA_DEVICE_MAX_CONNECTIONS hardware queues, eight unless the process says
+// otherwise, and kernels behind a resident one in the same queue wait for it.
+// 1500-column problems on 8 SMs each: 8 in 50 ms, 9 in 75 ms, 16 in 171 ms; two
+// rounds of eight on 17 SMs take 68 ms.
+int resident_streams() {
+    const char* v = std::getenv("CUDA_DEVICE_MAX_CONNECTIONS");
+    const int n = v ? std::atoi(v) : 0;
+    return n >= 1 && n <= 32 ? n : 8;
+}
 
 // Work of a problem's level, in FP64 operations of the resident kernel: the
 // sweeps of a basis that grows with the columns (n k each, k about an eighth
@@ -54,33 +60,56 @@ double cost_estimate(const DeviceOperator& op) {
     return 4.0 * op.rows() * n;
 }
 
-// SMs of each problem in LPT order, from the batch alone (so that a repeat
-// gives the same sums): of the `workers` problems that run from position p
-// on, each takes the part of the SMs that the square root of its work is of
-// theirs (which makes the sum of work / SMs smallest; in proportion to the
-// work the 16 problems take as long with 8 in flight, 128 ms, and 147 instead
-// of 129 ms with 4).  A tenth of the SMs stays free for the checkpoints'
-// kernels, which find no room beside a resident block.
+// SMs of each problem in LPT order (0: it has no resident levels), from the
+// batch alone (so that a repeat gives the same sums): of the `at_once` resident
+// problems that run from position p on, each takes the part of the SMs that the
+// square root of its work is of theirs (which makes the sum of work / SMs
+// smallest; in proportion to the work the 16 problems took as long with 8 in
+// flight, 128 ms, and 147 instead of 129 ms with 4).  A tenth of the SMs stays
+// free for the checkpoints' kernels, which find no room beside a resident block.
 std::vector<int> sm_shares(const std::vector<BatchItem>& items, const std::vector<int>& order,
-                           int workers) {
-    const int count = (int)order.size(), sms = sm_count();
-    std::vector<double> weight(count, 0.0);
-    for (int p = 0; p < count; ++p) {
+                           int at_once) {
+    const int sms = sm_count();
+    std::vector<int> at;  // positions with resident levels
+    std::vector<double> weight;
+    for (int p = 0; p < (int)order.size(); ++p) {
         ResidentOperator view;
         const DeviceOperator& op = *items[order[p]].op;
-        if (resident_levels(op, &view)) weight[p] = std::sqrt(cost_estimate(op));
+        if (!resident_levels(op, &view)) continue;
+        at.push_back(p);
+        weight.push_back(std::sqrt(cost_estimate(op)));
     }
-    std::vector<int> share(count, 0);
+    const int count = (int)at.size();
+    std::vector<int> share(order.size(), 0);
     for (int p = 0; p < count; ++p) {
-        // the last `workers` problems run beside each other to the end
-        const int first = std::max(0, std::min(p, count - workers));
+        // the last `at_once` problems run beside each other to the end
+        const int first = std::max(0, std::min(p, count - at_once));
         double sum = 0.0;
-        for (int q = first; q < std::min(count, first + workers); ++q) sum += weight[q];
-        if (weight[p] > 0.0)
-            share[p] = std::clamp((int)(0.9 * sms * weight[p] / sum), kMinShare, sms);
+        for (int q = first; q < std::min(count, first + at_once); ++q) sum += weight[q];
+        share[at[p]] = std::clamp((int)(0.9 * sms * weight[p] / sum), kMinShare, sms);
     }
     return share;
 }
+
+// The problems in LPT order; position -1: nothing is left for this worker.
+class Queue {
+public:
+    explicit Queue(const std::vector<int>& share) : share_(share), taken_(share.size(), false) {}
+    int take(bool resident_too) {
+        std::lock_guard<std::mutex> lock(mu_);
+        for (int p = 0; p < (int)share_.size(); ++p) {
+            if (taken_[p] || (share_[p] > 0 && !resident_too)) continue;
+            taken_[p] = true;
+            return p;
+        }
+        return -1;
+    }
+
+private:
+    const std::vector<int>& share_;
+    std::vector<bool> taken_;
+    std::mutex mu_;
+};
 
 }  // namespace
 
@@ -105,11 +134,6 @@ std::vector<BatchOutcome> solve_amfls_batch(const std::vector<BatchItem>& items,
             throw std::invalid_argument("each problem of a batch needs its own operator");
     }
     workers = std::min(workers, count);
-    const bool resident = std::all_of(items.begin(), items.end(), [](const BatchItem& it) {
-        ResidentOperator view;
-        return resident_levels(*it.op, &view);
-    });
-    if (resident) workers = std::min(workers, kResidentStreams);
     std::vector<int> order(count);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
@@ -117,8 +141,12 @@ std::vector<BatchOutcome> solve_amfls_batch(const std::vector<BatchItem>& items,
     });
     int device = 0;
     AMFLS_CUDA(cudaGetDevice(&device));
-    const std::vector<int> share = sm_shares(items, order, workers);
-    std::atomic<int> next{0};
+    const int at_once = std::min(workers, resident_streams());
+    const std::vector<int> share = sm_shares(items, order, at_once);
+    // workers beyond `at_once` take the other problems alone, on streams of
+    // their own: the resident solves keep to as many streams as run at a time
+    workers = std::min(workers, at_once + (int)std::count(share.begin(), share.end(), 0));
+    Queue queue(share);
     const auto t0 = std::chrono::steady_clock::now();
     auto work = [&](int w) {
         cudaStream_t s = nullptr;
@@ -129,7 +157,7 @@ std::vector<BatchOutcome> solve_amfls_batch(const std::vector<BatchItem>& items,
             // the remaining problems are left to the other workers
             return;
         }
-        for (int k = next.fetch_add(1); k < count; k = next.fetch_add(1)) {
+        for (int k; (k = queue.take(w < at_once)) >= 0;) {
             const int i = order[k];
             BatchOutcome& o = out[i];
             o.worker = w;

@@ -367,8 +367,9 @@ int amfls_gpu_csr_operator_schedule(const amfls_gpu_operator* op, int* chains,
  * problems, problem i = (ops[i], d_b[i], options[i]) with its solution in
  * d_solutions[i] (a distinct operator per problem: an operator's products
  * use scratch it owns), solved concurrently by `workers` host threads with one
- * CUDA stream each (streams created and destroyed inside the call), at most
- * eight at a time when all are CSR problems, largest estimated work first.  results[i] as from
+ * CUDA stream each (streams created and destroyed inside the call), largest
+ * estimated work first; of the CSR problems at most CUDA_DEVICE_MAX_CONNECTIONS
+ * (eight when it is not set) run at a time. results[i] as from
  * amfls_gpu_solve_amfls (trace rows counted, not copied); seconds[i] (may be
  * NULL) the wall time of problem i; *wall_seconds (may be NULL) the whole
  * batch.  Returns the first problem's error if any solve raised (the others
