@@ -13,12 +13,13 @@ namespace amfls_gpu {
 // Host-side CUDA error check that turns a failure into an exception; the
 // C ABI layer converts it into an error code and a message.
 struct CudaError : std::runtime_error {
-    using std::runtime_error::runtime_error;
+    CudaError(const std::string& what, cudaError_t code) : std::runtime_error(what), code(code) {}
+    cudaError_t code;
 };
 
 inline void check_cuda(cudaError_t e, const char* what) {
     if (e != cudaSuccess) {
-        throw CudaError(std::string(what) + ": " + cudaGetErrorString(e));
+        throw CudaError(std::string(what) + ": " + cudaGetErrorString(e), e);
     }
 }
 

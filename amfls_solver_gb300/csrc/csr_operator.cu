@@ -580,17 +580,13 @@ constexpr double kTuneMargin = 0.10;
 constexpr double kVectorMargin = 0.05;
 
 // Operators of at most this many nonzeros carry the sliced-row copy that the
-// resident level kernel multiplies by (two sides of 12 bytes a nonzero, up to
-// a quarter more for padding: 4 GB at the limit), where it takes at most half
-// of the free memory.  It pays at every size measured, up to the 40 million
-// nonzeros of the 2M x 500k matrix; beyond the limit the kernel chain runs.
+// resident kernels multiply by (two sides of 12 bytes a nonzero, up to a
+// quarter more for padding: 4 GB at the limit, and 9 bytes a row and column),
+// where the memory for it is there.  It pays at every size measured, up to the
+// 40 million nonzeros of the 2M x 500k matrix; beyond the limit the kernel chain
+// runs.  What else is allocated does not count: the tables decide the order of a
+// solve's sums.
 constexpr long long kResidentMaxNonzeros = 1LL << 27;
-
-bool sliced_rows_fit(long long nnz) {
-    size_t free_bytes = 0, total = 0;
-    AMFLS_CUDA(cudaMemGetInfo(&free_bytes, &total));
-    return nnz <= kResidentMaxNonzeros && 2 * 30 * (size_t)nnz <= free_bytes;
-}
 
 struct CsrOperator::Side {
     long long* off = nullptr;  // count+1
@@ -829,7 +825,7 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
     AMFLS_CUDA(cudaMemsetAsync(w, 0, sizeof(Work), stream));
     int *lens = nullptr, *bins = nullptr, *row_of = nullptr, *perm = nullptr, *counts = nullptr;
     const long long big = std::max<long long>(1, std::max<long long>(rows_, cols_));
-    AMFLS_CUDA(cudaMallocAsync(&lens, sizeof(int) * big, stream));
+    AMFLS_CUDA(cudaMallocAsync(&lens, sizeof(int) * ((size_t)rows_ + cols_), stream));
     AMFLS_CUDA(cudaMallocAsync(&bins, sizeof(int) * big, stream));
     AMFLS_CUDA(cudaMallocAsync(&row_of, sizeof(int) * std::max<long long>(1, nnz), stream));
     AMFLS_CUDA(cudaMallocAsync(&perm, sizeof(int) * std::max<long long>(1, nnz), stream));
@@ -862,11 +858,6 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
     AMFLS_CUDA(cudaStreamSynchronize(stream));
     if (err & 4) fail("CSR column index is out of range");
     if (err & 8) fail("CSR values must be finite");
-    const bool sliced_rows = sliced_rows_fit(nnz);
-    if (sliced_rows)
-        sliced::build(A.rows, A.off, A.idx, A.val, lens, rows_, sliced::elements_per_lane(nnz),
-                      stream);
-
     // transpose: stable sort of entry ids by column
     AMFLS_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (cols_ + 1), stream));
     if (nnz > 0) {
@@ -912,13 +903,9 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
 
     // transpose bins
     check_offsets_kernel<<<setup_grid(cols_), 256, 0, stream>>>(
-        T.off, cols_, nnz, &w->err, &w->max_len_c, lens, elems_per_lane_, bins);
+        T.off, cols_, nnz, &w->err, &w->max_len_c, lens + rows_, elems_per_lane_, bins);
     AMFLS_LAUNCHED();
     build_bins(T, bins, stream);
-    if (sliced_rows)
-        sliced::build(T.rows, T.off, T.idx, T.val, lens, cols_, sliced::elements_per_lane(nnz),
-                      stream);
-
     // int32 offsets and tilings of both sides for the streamed products
     for (Side* sd : {&A, &T}) {
         narrow_offsets_kernel<<<setup_grid(sd->count + 1), 256, 0, stream>>>(sd->off, sd->count,
@@ -957,12 +944,34 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
 
     AMFLS_CUDA(cudaFreeAsync(frob_partials, stream));
     AMFLS_CUDA(cudaFreeAsync(w, stream));
-    AMFLS_CUDA(cudaFreeAsync(lens, stream));
     AMFLS_CUDA(cudaFreeAsync(bins, stream));
     AMFLS_CUDA(cudaFreeAsync(row_of, stream));
     AMFLS_CUDA(cudaFreeAsync(perm, stream));
     AMFLS_CUDA(cudaFreeAsync(counts, stream));
+    // last, when all that the operator must have is there
+    try {
+        build_sliced_rows(lens, lens + rows_, stream);
+    } catch (...) {
+        stream_free(lens, stream);
+        throw;
+    }
+    AMFLS_CUDA(cudaFreeAsync(lens, stream));
     AMFLS_CUDA(cudaStreamSynchronize(stream));
+}
+
+// The tables of both sides, or none where the memory runs out.
+void CsrOperator::build_sliced_rows(const int* row_lens, const int* col_lens, cudaStream_t stream) {
+    if (nnz_ > kResidentMaxNonzeros) return;
+    const int per_lane = sliced::elements_per_lane(nnz_);
+    try {
+        sliced::build(a_->rows, a_->off, a_->idx, a_->val, row_lens, rows_, per_lane, stream);
+        sliced::build(t_->rows, t_->off, t_->idx, t_->val, col_lens, cols_, per_lane, stream);
+    } catch (const CudaError& e) {
+        a_->rows.release();
+        t_->rows.release();
+        if (e.code != cudaErrorMemoryAllocation) throw;
+        cudaGetLastError();  // the failed allocation's
+    }
 }
 
 namespace {

@@ -53,6 +53,7 @@ private:
     struct Side;
     void build(const long long* d_off, const long long* d_idx, const double* d_val,
                cudaStream_t stream);
+    void build_sliced_rows(const int* row_lens, const int* col_lens, cudaStream_t stream);
     void build_bins(Side& s, const int* d_bins, cudaStream_t stream);
     void tune_single_column(Side& s, const std::vector<long long>& host_off,
                             cudaStream_t stream);
