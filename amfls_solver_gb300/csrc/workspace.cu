@@ -959,7 +959,8 @@ __global__ void scale_copy_kernel(const double* src, double* dst, long long n, d
 //   |z_j| = 1 / |rho_j| + |theta_j / rho_j| |z_{j-1}|.
 // rhobar takes the sign of alpha's product so far (a damping rotation makes it
 // positive first).  Tiles with an entry outside 1e-15 .. 1e15 (a zero beta
-// apart) could leave FP64's range in the ratio: they are rotated one by one.
+// apart) could leave FP64's range in the ratio, and for lambda = 0 tiles whose 1 / q
+// passes 1e300 have left it: they are rotated one by one.
 constexpr int kProjThreads = 128;
 constexpr int kProjTile = 512;
 
@@ -1007,39 +1008,8 @@ projected_solve_kernel(const double* alpha, const double* beta, const double* g,
             B[i] = lambda > 0.0 ? a2 : 1.0 / a2;
             negative[i] = alpha[j] < 0.0 ? 1 : 0;
         }
-        if (__syncthreads_or(unsafe)) {  // one thread, rotation by rotation
-            if (tid == 0) {
-                double c = c_s, s = s_s, phibar = phibar_s;
-                const double root = sqrt(lambda);
-                for (int j = j0; j < j0 + nt; ++j) {
-                    // the rotation of column j-1 acting on rows (j-1, j) meets column j
-                    theta[j] = s * alpha[j];
-                    double rhobar = c * alpha[j];
-                    if (lambda > 0.0) {
-                        const double r = hypot(rhobar, root);
-                        phibar = rhobar / r * phibar;
-                        rhobar = r;
-                    }
-                    c = 1.0;
-                    s = 0.0;
-                    rho[j] = rhobar;
-                    phi[j] = phibar;
-                    if (j + 1 < rows_t) {
-                        const double b = beta[j];
-                        const double r = hypot(rhobar, b);
-                        c = rhobar / r;
-                        s = b / r;
-                        rho[j] = r;
-                        phi[j] = c * phibar + s * g[j + 1];
-                        phibar = -s * phibar + c * g[j + 1];
-                    }
-                }
-                c_s = c;
-                s_s = s;
-                phibar_s = phibar;
-            }
-            __syncthreads();
-        } else {
+        bool chained = !__syncthreads_or(unsafe);
+        if (chained) {
             if (tid == 0) {  // the chain of q
                 if (lambda > 0.0) {
                     double x = rhobar0 * rhobar0, w = 1.0;
@@ -1077,7 +1047,48 @@ projected_solve_kernel(const double* alpha, const double* beta, const double* g,
                         negative[i] = (signed char)neg;
                     }
             }
+            // 1 / q of columns whose beta exceeds alpha again and again grows past
+            // FP64's range: then rhobar, its root, is taken column by column
+            int spilled = 0;
             __syncthreads();
+            if (!(lambda > 0.0))
+                for (int i = tid; i < nt; i += kProjThreads)
+                    if (!(X[i] < 1e300)) spilled = 1;
+            chained = !__syncthreads_or(spilled);
+        }
+        if (!chained) {  // one thread, rotation by rotation
+            if (tid == 0) {
+                double c = c_s, s = s_s, phibar = phibar_s;
+                const double root = sqrt(lambda);
+                for (int j = j0; j < j0 + nt; ++j) {
+                    // the rotation of column j-1 acting on rows (j-1, j) meets column j
+                    theta[j] = s * alpha[j];
+                    double rhobar = c * alpha[j];
+                    if (lambda > 0.0) {
+                        const double r = hypot(rhobar, root);
+                        phibar = rhobar / r * phibar;
+                        rhobar = r;
+                    }
+                    c = 1.0;
+                    s = 0.0;
+                    rho[j] = rhobar;
+                    phi[j] = phibar;
+                    if (j + 1 < rows_t) {
+                        const double b = beta[j];
+                        const double r = hypot(rhobar, b);
+                        c = rhobar / r;
+                        s = b / r;
+                        rho[j] = r;
+                        phi[j] = c * phibar + s * g[j + 1];
+                        phibar = -s * phibar + c * g[j + 1];
+                    }
+                }
+                c_s = c;
+                s_s = s;
+                phibar_s = phibar;
+            }
+            __syncthreads();
+        } else {
             for (int i = tid; i < nt; i += kProjThreads) {
                 const int j = j0 + i;
                 const double sign = negative[i] ? -1.0 : 1.0;
