@@ -300,17 +300,38 @@ __device__ void cta_qr(double* A, int rows, int nf, int nt, int lda, double* red
 // kSmallQrThreads threads): eight lanes a column, every warp recomputes the
 // reflector, and one block barrier per column is left (64 levels of 8 columns,
 // with the back substitution: 4.9 -> 2.6 ms).  H = I - g v v^T with
-// v = (x0 - beta, x1, ...) and g = 1 / (||x|| (||x|| + |x0|)).
+// v = (x0 - beta, x1, ...) and g = 1 / (||x|| (||x|| + |x0|)); where the squares
+// come near the ends of FP64's range, g would pass them, and v is scaled to
+// v_0 = 1 as in cta_qr.
 constexpr int kSmallQrThreads = 128;
 
-__device__ void small_qr(double* A, int rows, int nf, int nt, int lda) {
+// A[:, j+1 : nt] -= g v (v^T A): v_j = v0, v_i = v(i) below it.
+template <typename V>
+__device__ __forceinline__ void small_reflect(double* A, int rows, int j, int nt, int lda,
+                                              double v0, double g, V&& v) {
     const int sub = threadIdx.x & 7, group = threadIdx.x >> 3;
+    for (int l0 = j + 1; l0 < nt; l0 += kSmallQrThreads / 8) {
+        const int l = l0 + group;
+        double* cl = A + (long long)min(l, nt - 1) * lda;
+        double w = sub == 0 ? v0 * cl[j] : 0.0;
+        for (int i = j + 1 + sub; i < rows; i += 8) w = fma(v(i), cl[i], w);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+        w *= g;
+        if (l < nt) {
+            if (sub == 0) cl[j] = fma(-w, v0, cl[j]);
+            for (int i = j + 1 + sub; i < rows; i += 8) cl[i] = fma(-w, v(i), cl[i]);
+        }
+    }
+}
+
+__device__ void small_qr(double* A, int rows, int nf, int nt, int lda) {
+    const int sub = threadIdx.x & 7;
     const bool active = threadIdx.x < kSmallQrThreads;
     const int steps = min(nf, rows);
     double beta = 0.0;
     for (int j = 0; j < steps; ++j) {
         double* col = A + (long long)j * lda;
-        bool reflects = false;
         if (active) {
             double sigma = 0.0;
             for (int i = j + 1 + sub; i < rows; i += 8) sigma = fma(col[i], col[i], sigma);
@@ -318,30 +339,26 @@ __device__ void small_qr(double* A, int rows, int nf, int nt, int lda) {
             for (int o = 4; o > 0; o >>= 1) sigma += __shfl_xor_sync(0xffffffffu, sigma, o);
             const double x0 = col[j];
             beta = x0;
-            reflects = sigma != 0.0;
-            if (reflects) {  // the same in every thread
-                const double sq = fma(x0, x0, sigma), rn = rsqrt(sq), nrm = sq * rn;
-                beta = x0 >= 0.0 ? -nrm : nrm;
-                const double g = rn / (nrm + fabs(x0)), v0 = x0 - beta;
-                for (int l0 = j + 1; l0 < nt; l0 += kSmallQrThreads / 8) {
-                    const int l = l0 + group;
-                    double* cl = A + (long long)min(l, nt - 1) * lda;
-                    double w = sub == 0 ? v0 * cl[j] : 0.0;
-                    for (int i = j + 1 + sub; i < rows; i += 8) w = fma(col[i], cl[i], w);
-#pragma unroll
-                    for (int o = 4; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-                    w *= g;
-                    if (l < nt) {
-                        if (sub == 0) cl[j] = fma(-w, v0, cl[j]);
-                        for (int i = j + 1 + sub; i < rows; i += 8) cl[i] = fma(-w, col[i], cl[i]);
-                    }
+            if (sigma != 0.0) {  // the same in every thread
+                const double sq = fma(x0, x0, sigma);
+                if (sq > 1e-280 && sq < 1e280) {
+                    const double rn = rsqrt(sq), nrm = sq * rn;
+                    beta = x0 >= 0.0 ? -nrm : nrm;
+                    small_reflect(A, rows, j, nt, lda, x0 - beta, rn / (nrm + fabs(x0)),
+                                  [&](int i) { return col[i]; });
+                } else {
+                    const double nrm = sqrt(sq);
+                    beta = x0 >= 0.0 ? -nrm : nrm;
+                    const double scale = 1.0 / (x0 - beta);
+                    small_reflect(A, rows, j, nt, lda, 1.0, (beta - x0) / beta,
+                                  [&](int i) { return col[i] * scale; });
                 }
             }
         }
         __syncthreads();
         // nobody reads the column again
         if (threadIdx.x == 0) col[j] = beta;
-        if (active && reflects)
+        if (active)
             for (int i = j + 1 + (int)threadIdx.x; i < rows; i += kSmallQrThreads) col[i] = 0.0;
     }
     __syncthreads();
