@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("width", [1, 2, 5, 15])
-@pytest.mark.parametrize("exponent", [-520, -518, -516, -514, -505, -480, -300, 300, 480, 508])
+@pytest.mark.parametrize("exponent", [-518, -516, -514, -505, -480, -300, 300, 480, 508])
 def test_scaled_blocks_solve_the_same_problem(width, exponent):
     import amfls_solver_gb300 as amfls
 
@@ -26,7 +26,7 @@ def test_scaled_blocks_solve_the_same_problem(width, exponent):
     b = p.matvec(x)
     p.values = np.ldexp(p.values, exponent)
     r = amfls.run_fixed_rbgk(csr_tensor(p), torch.from_numpy(b).cuda(), auxiliary_width=width,
-                             tolerance=1e-9)
+                             maximum_depth=60, tolerance=1e-9)
     # a certified solve, or the full basis where the certificate's own squares underflow
     assert r.status in (0, 2)
     got = np.ldexp(r.solution.cpu().numpy(), exponent)
