@@ -84,9 +84,11 @@ __global__ void bin_rows_kernel(const int* bins, int rows, int* ids, int* counts
     __shared__ int local[kLengthBins];
     if (threadIdx.x < kLengthBins) local[threadIdx.x] = 0;
     __syncthreads();
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
+    // 64 bits: rows may end within a stride of 2^31
+    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < rows;
+         r += (long long)gridDim.x * blockDim.x) {
         atomicAdd(&local[bins[r]], 1);
-        ids[r] = r;
+        ids[r] = (int)r;
     }
     __syncthreads();
     if (threadIdx.x < kLengthBins && local[threadIdx.x])

@@ -17,9 +17,11 @@ __global__ void count_groups_kernel(const int* lens, int count, int per_lane, in
     __shared__ int local[6];
     if (threadIdx.x < 6) local[threadIdx.x] = 0;
     __syncthreads();
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < count; r += gridDim.x * blockDim.x) {
+    // 64 bits: rows and tasks may end within a stride of 2^31
+    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < count;
+         r += (long long)gridDim.x * blockDim.x) {
         atomicAdd(&local[5 - lane_shift(lens[r], per_lane)], 1);
-        rows_of[r] = r;
+        rows_of[r] = (int)r;
     }
     __syncthreads();
     if (threadIdx.x < 6 && local[threadIdx.x]) atomicAdd(&counts[threadIdx.x], local[threadIdx.x]);
@@ -31,7 +33,8 @@ struct Groups {
 };
 
 __global__ void task_steps_kernel(Groups g, const int* sorted_lens, int ntasks, int* steps) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= ntasks; t += gridDim.x * blockDim.x) {
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t <= ntasks;
+         t += (long long)gridDim.x * blockDim.x) {
         if (t == ntasks) {
             steps[t] = 0;
             continue;
@@ -39,7 +42,7 @@ __global__ void task_steps_kernel(Groups g, const int* sorted_lens, int ntasks, 
         int i = 0;
         while (t >= g.task_start[i + 1]) ++i;
         const int shift = 5 - i;
-        const int first = g.row_start[i] + (t - g.task_start[i]) * (32 >> shift);
+        const int first = g.row_start[i] + (int)(t - g.task_start[i]) * (32 >> shift);
         steps[t] = (sorted_lens[first] + (1 << shift) - 1) >> shift;
     }
 }
@@ -48,19 +51,21 @@ __global__ void fill_kernel(Groups g, const int* rows, const int* sorted_lens, c
                             int ntasks, const long long* off, const int* idx, const double* val,
                             int2* tasks, int2* lanes, int* out_idx, double* out_val) {
     const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntasks; t += warps) {
+    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; t < ntasks;
+         t += warps) {
         int i = 0;
         while (t >= g.task_start[i + 1]) ++i;
         const int shift = 5 - i, sub = lane & ((1 << shift) - 1);
-        const int pos = g.row_start[i] + (t - g.task_start[i]) * (32 >> shift) + (lane >> shift);
+        const long long pos =
+            g.row_start[i] + (t - g.task_start[i]) * (32 >> shift) + (lane >> shift);
         const bool has = pos < g.row_start[i + 1];
         const int row = has ? rows[pos] : -1;
         const int len = has ? sorted_lens[pos] : 0;
         const int n = len > sub ? (len - sub + (1 << shift) - 1) >> shift : 0;
         const int s0 = first[t], steps = first[t + 1] - s0;
         if (lane == 0) tasks[t] = make_int2(s0, steps);
-        lanes[(long long)t * 32 + lane] = make_int2(row, n);
+        lanes[t * 32 + lane] = make_int2(row, n);
         const long long e0 = has ? off[row] + sub : 0;
         for (int j = 0; j < steps; ++j) {
             const long long o = ((long long)s0 + j) * 32 + lane;
@@ -104,8 +109,8 @@ void build(Store& store, const long long* off, const int* idx, const double* val
         AMFLS_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, bytes, lens, lens_out, rows,
                                                              sorted, count, 0, 31, stream));
         // at most one partly filled task per group beyond count / 1 tasks
-        AMFLS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, steps, first, count + 7,
-                                                 stream));
+        AMFLS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, steps, first,
+                                                 (int)std::min(count + 7LL, 0x7fffffffLL), stream));
         bytes = std::max({bytes, scan_bytes, (size_t)1});
         AMFLS_CUDA(cudaMallocAsync(&tmp, bytes, stream));
         AMFLS_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp, bytes, lens, lens_out, rows,
@@ -117,11 +122,11 @@ void build(Store& store, const long long* off, const int* idx, const double* val
         for (int i = 0; i < 6; ++i) {
             const int per = 1 << i;  // rows per task: 32 / (32 >> i)
             g.row_start[i + 1] = g.row_start[i] + host[i];
-            g.task_start[i + 1] = g.task_start[i] + (host[i] + per - 1) / per;
+            g.task_start[i + 1] = g.task_start[i] + (int)((host[i] + (long long)per - 1) / per);
         }
         const int ntasks = g.task_start[6];
-        stream_alloc(&steps, sizeof(int) * (ntasks + 1), stream);
-        stream_alloc(&first, sizeof(int) * (ntasks + 1), stream);
+        stream_alloc(&steps, sizeof(int) * (ntasks + 1LL), stream);
+        stream_alloc(&first, sizeof(int) * (ntasks + 1LL), stream);
         task_steps_kernel<<<grid_for(ntasks + 1), 256, 0, stream>>>(g, lens_out, ntasks, steps);
         AMFLS_LAUNCHED();
         AMFLS_CUDA(cub::DeviceScan::ExclusiveSum(tmp, bytes, steps, first, ntasks + 1, stream));
