@@ -79,13 +79,13 @@ __device__ __forceinline__ double warp_sums(double (&v)[N], int& index) {
     return v[0];
 }
 
-// A(o, i) at a[o * ld + i] (i contiguous): a warp owns dot_outputs(S) outputs
-// and strides i across its lanes.
-template <int S>
+// A(o, i) at a[o * ld + i] (i contiguous): a warp owns J outputs and strides i
+// across its lanes.
+template <int S, int J>
 __global__ void __launch_bounds__(kThreads)
 dot_block_kernel(const double* __restrict__ a, long long ld, int outer, int inner, int chunk,
                  const double* __restrict__ x, long long ldx, double* partial, const int* guard) {
-    constexpr int J = dot_outputs(S), N = pow2_ceil(J * S);
+    constexpr int N = pow2_ceil(J * S);
     if (guard && *guard == 0) return;
     const int lane = threadIdx.x & 31;
     const long long o0 = ((long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * J;
@@ -145,60 +145,68 @@ across_block_kernel(const double* __restrict__ a, long long ld, int outer, int i
 // thread each 32nd chunk of one of them, and the slices are added in a fixed
 // tree; else a thread adds all of one output's.  A thread per output took 52
 // to 107 us for 512 outputs of 512 chunks, a chain of dependent loads and
-// additions (sliced 5 to 12 us), and is the faster one where the outputs fill the
-// SM quarters with warps (65536 outputs of 16 chunks: 6.2 against 14.2 us).
-constexpr int kSlicedChunks = 16, kSliceOutputs = 8;
+// additions (sliced 5 to 12 us); sliced, the additions over the slices are the
+// outputs' own, 0.5 us per 1000.  Whole products, us, plain and sliced, by outputs a
+// chunk: 128 (4096 of 32) 15.3 and 14.8, (16384 of 128) 134.8 and 131.0; 205 (4096 of
+// 20) 11.8 and 12.1; 256 (8192 of 32) 20.9 and 22.8, (16384 of 64) 66.5 and 70.0, (32768 of
+// 128) 249 and 257.
+constexpr int kSlicedChunks = 16, kSliceOutputs = 8, kSlicedPerChunk = 150;
+inline bool sliced_sums(long long outputs, int chunks) {
+    return chunks >= kSlicedChunks && outputs <= (long long)kSlicedPerChunk * chunks;
+}
 
-template <bool kSliced>
+__global__ void reduce_block_kernel(const double* partial, int chunks, int S, int outer, double* y,
+                                    long long ldy, const int* guard) {
+    if (guard && *guard == 0) return;
+    const long long total = (long long)S * outer;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+         t += (long long)gridDim.x * blockDim.x) {
+        const int c = (int)(t / outer);
+        const long long o = t % outer;
+        double s = 0.0;
+        for (int ch = 0; ch < chunks; ++ch) s += partial[((long long)ch * S + c) * outer + o];
+        y[o + c * ldy] = s;
+    }
+}
+
 __global__ void __launch_bounds__(kThreads)
-reduce_block_kernel(const double* __restrict__ partial, int chunks, int S, int outer, double* y,
-                    long long ldy, const int* guard) {
+reduce_sliced_kernel(const double* __restrict__ partial, int chunks, int S, int outer, double* y,
+                     long long ldy, const int* guard) {
     __shared__ double slice[kThreads / 32][kSliceOutputs];
     if (guard && *guard == 0) return;
     const long long total = (long long)S * outer;
-    auto put = [&](long long t, double v) {
-        const int c = (int)(t / outer);
-        y[t - (long long)c * outer + c * ldy] = v;
-    };
-    if constexpr (kSliced) {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        constexpr int kSlices = kThreads / kSliceOutputs;
-        for (long long t0 = (long long)blockIdx.x * kSliceOutputs; t0 < total;
-             t0 += (long long)gridDim.x * kSliceOutputs) {
-            const long long t = t0 + lane % kSliceOutputs;
-            double x[4] = {0.0, 0.0, 0.0, 0.0};
-            if (t < total) {
-                const double* p = partial + t;
-                int ch = threadIdx.x / kSliceOutputs;
-                for (; ch + 3 * kSlices < chunks; ch += 4 * kSlices) {
-                    double v[4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kSlices = kThreads / kSliceOutputs;
+    for (long long t0 = (long long)blockIdx.x * kSliceOutputs; t0 < total;
+         t0 += (long long)gridDim.x * kSliceOutputs) {
+        const long long t = t0 + lane % kSliceOutputs;
+        double x[4] = {0.0, 0.0, 0.0, 0.0};
+        if (t < total) {
+            const double* p = partial + t;
+            int ch = threadIdx.x / kSliceOutputs;
+            for (; ch + 3 * kSlices < chunks; ch += 4 * kSlices) {
+                double v[4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) v[u] = p[(ch + u * kSlices) * total];
+                for (int u = 0; u < 4; ++u) v[u] = p[(ch + u * kSlices) * total];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) x[u] += v[u];
-                }
-#pragma unroll
-                for (int u = 0; u < 3; ++u)
-                    if (ch + u * kSlices < chunks) x[u] += p[(ch + u * kSlices) * total];
+                for (int u = 0; u < 4; ++u) x[u] += v[u];
             }
-            double v = (x[0] + x[1]) + (x[2] + x[3]);
-            v += __shfl_xor_sync(0xffffffffu, v, 8);
-            v += __shfl_xor_sync(0xffffffffu, v, 16);
-            if (lane < kSliceOutputs) slice[warp][lane] = v;
-            __syncthreads();
-            if (threadIdx.x < kSliceOutputs && t < total)
-                put(t, ((slice[0][lane] + slice[1][lane]) + (slice[2][lane] + slice[3][lane])) +
-                           ((slice[4][lane] + slice[5][lane]) +
-                            (slice[6][lane] + slice[7][lane])));
-            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < 3; ++u)
+                if (ch + u * kSlices < chunks) x[u] += p[(ch + u * kSlices) * total];
         }
-    } else {
-        for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-             t += (long long)gridDim.x * blockDim.x) {
-            double s = partial[t];
-            for (int ch = 1; ch < chunks; ++ch) s += partial[ch * total + t];
-            put(t, s);
+        double v = (x[0] + x[1]) + (x[2] + x[3]);
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        v += __shfl_xor_sync(0xffffffffu, v, 16);
+        if (lane < kSliceOutputs) slice[warp][lane] = v;
+        __syncthreads();
+        if (threadIdx.x < kSliceOutputs && t < total) {
+            const int c = (int)(t / outer);
+            y[t - (long long)c * outer + c * ldy] =
+                ((slice[0][lane] + slice[1][lane]) + (slice[2][lane] + slice[3][lane])) +
+                ((slice[4][lane] + slice[5][lane]) + (slice[6][lane] + slice[7][lane]));
         }
+        __syncthreads();
     }
 }
 
@@ -397,44 +405,59 @@ int grid_1d(long long items) {
     return (int)std::max<long long>(1, std::min<long long>(target_blocks(), (items + 255) / 256));
 }
 
-// chunking for the block kernels: enough blocks to fill the GPU twice over
-// (J: outputs of a warp of the dot kernel)
-void block_chunks(bool dot, int J, int out_n, int in_n, int& blocks_x, int& chunks, int& chunk) {
+// How a product is split: enough blocks to fill the GPU twice over.
+struct Split {
+    int J;  // outputs of a warp of the dot kernel
+    int blocks_x, chunks, chunk;
+};
+
+Split split_of(bool dot, int J, int min_rows, int out_n, int in_n) {
+    Split p{J, 0, 0, 0};
     if (dot) {
         const long long groups = ((long long)out_n + J - 1) / J;
-        blocks_x = (int)((groups + kThreads / 32 - 1) / (kThreads / 32));
+        p.blocks_x = (int)((groups + kThreads / 32 - 1) / (kThreads / 32));
     } else {
-        blocks_x = (out_n + kThreads - 1) / kThreads;
+        p.blocks_x = (out_n + kThreads - 1) / kThreads;
     }
-    const int min_rows = dot ? 512 : 32;
-    chunks = std::max(1, std::min((2 * target_blocks() + blocks_x - 1) / blocks_x,
-                                  (in_n + min_rows - 1) / min_rows));
-    chunk = (in_n + chunks - 1) / chunks;
-    chunks = (in_n + chunk - 1) / chunk;
+    p.chunks = std::max(1, std::min((2 * target_blocks() + p.blocks_x - 1) / p.blocks_x,
+                                    (in_n + min_rows - 1) / min_rows));
+    p.chunk = (in_n + p.chunks - 1) / p.chunks;
+    p.chunks = (in_n + p.chunk - 1) / p.chunk;
+    return p;
+}
+
+// of a block product of S columns
+Split block_split(bool dot, int S, int out_n, int in_n) {
+    if (!dot) return split_of(false, 1, 32, out_n, in_n);
+    return split_of(true, dot_outputs(S), 512, out_n, in_n);
+}
+
+// of a double-double product
+Split refined_split(bool dot, int out_n, int in_n) {
+    return split_of(dot, 1, dot ? 512 : 32, out_n, in_n);
 }
 
 template <int S>
 void launch_block(bool dot, const double* a, long long ld, int out_n, int in_n, const double* x,
                   long long ldx, double* partial, double* y, long long ldy, cudaStream_t s,
                   const int* guard = nullptr, bool slices = true) {
-    int blocks_x = 0, chunks = 0, chunk = 0;
-    block_chunks(dot, dot_outputs(S), out_n, in_n, blocks_x, chunks, chunk);
-    const dim3 grid(blocks_x, chunks);
-    if (dot)
-        dot_block_kernel<S><<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, chunk, x, ldx, partial,
-                                                       guard);
-    else
-        across_block_kernel<S><<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, chunk, x, ldx,
+    const Split p = block_split(dot, S, out_n, in_n);
+    const dim3 grid(p.blocks_x, p.chunks);
+    if (!dot)
+        across_block_kernel<S><<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, p.chunk, x, ldx,
                                                           partial, guard);
+    else
+        dot_block_kernel<S, dot_outputs(S)><<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, p.chunk,
+                                                                       x, ldx, partial, guard);
     AMFLS_LAUNCHED();
     const long long total = (long long)S * out_n;
-    if (slices && chunks >= kSlicedChunks && total <= 32LL * 4 * sm_count()) {
+    if (slices && sliced_sums(total, p.chunks)) {
         const long long groups = (total + kSliceOutputs - 1) / kSliceOutputs;
-        reduce_block_kernel<true><<<(int)std::min<long long>(groups, target_blocks()), kThreads, 0,
-                                    s>>>(partial, chunks, S, out_n, y, ldy, guard);
+        reduce_sliced_kernel<<<(int)std::min<long long>(groups, target_blocks()), kThreads, 0, s>>>(
+            partial, p.chunks, S, out_n, y, ldy, guard);
     } else {
-        reduce_block_kernel<false><<<grid_1d(total), kThreads, 0, s>>>(partial, chunks, S, out_n,
-                                                                       y, ldy, guard);
+        reduce_block_kernel<<<grid_1d(total), kThreads, 0, s>>>(partial, p.chunks, S, out_n, y, ldy,
+                                                                guard);
     }
     AMFLS_LAUNCHED();
 }
@@ -442,11 +465,11 @@ void launch_block(bool dot, const double* a, long long ld, int out_n, int in_n, 
 void launch_refined(bool dot, const double* a, long long ld, int out_n, int in_n,
                     const double* x_hi, const double* x_lo, double* partial, double* y_hi,
                     double* y_lo, int* finite, cudaStream_t s) {
-    int blocks_x = 0, chunks = 0, chunk = 0;
-    block_chunks(dot, 1, out_n, in_n, blocks_x, chunks, chunk);
-    const dim3 grid(blocks_x, chunks);
+    const Split p = refined_split(dot, out_n, in_n);
+    const int chunks = p.chunks;
+    const dim3 grid(p.blocks_x, chunks);
     double2* pairs = reinterpret_cast<double2*>(partial);
-    (dot ? dd_dot_kernel : dd_across_kernel)<<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, chunk,
+    (dot ? dd_dot_kernel : dd_across_kernel)<<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, p.chunk,
                                                                        x_hi, x_lo, pairs);
     AMFLS_LAUNCHED();
     // additions in a row on each SM quarter: `chunks` for every 32 outputs with a
@@ -488,13 +511,11 @@ DenseOperator::DenseOperator(int rows, int cols, const double* d_values, bool co
         for (int tr = 0; tr < 2; ++tr) {  // both directions, up to 8 columns per pass
             const int on = tr ? cols : rows, inn = tr ? rows : cols;
             const bool dot = column_major == (tr == 1);
-            int bx = 0, ch = 0, ck = 0;
-            for (int S = 1; S <= 8; ++S) {
-                block_chunks(dot, dot_outputs(S), on, inn, bx, ch, ck);
-                partial_cap_ = std::max(partial_cap_, (long long)S * ch * on);
-            }
-            block_chunks(dot, 1, on, inn, bx, ch, ck);  // double-double pairs
-            partial_cap_ = std::max(partial_cap_, 2LL * ch * on);
+            for (int S = 1; S <= 8; ++S)
+                partial_cap_ = std::max(partial_cap_,
+                                        (long long)S * block_split(dot, S, on, inn).chunks * on);
+            // double-double pairs
+            partial_cap_ = std::max(partial_cap_, 2LL * refined_split(dot, on, inn).chunks * on);
         }
         AMFLS_CUDA(cudaMalloc(&partials_,
                               sizeof(double) * std::max<long long>(1, partial_cap_)));
@@ -505,12 +526,12 @@ DenseOperator::DenseOperator(int rows, int cols, const double* d_values, bool co
         model_outer_kernel<<<og, kThreads, 0, stream>>>(a_, outer, inner, w, w + 9 + ig,
                                                         counter_ + 2, w + 8);
         AMFLS_LAUNCHED();
-        int bx = 0, chunks = 0, chunk = 0;
-        block_chunks(false, 1, inner, outer, bx, chunks, chunk);
+        const Split p = refined_split(false, inner, outer);
         double2* sums = reinterpret_cast<double2*>(partials_);
-        model_chunk_kernel<<<dim3(bx, chunks), kThreads, 0, stream>>>(a_, outer, inner, chunk, sums);
+        model_chunk_kernel<<<dim3(p.blocks_x, p.chunks), kThreads, 0, stream>>>(a_, outer, inner,
+                                                                               p.chunk, sums);
         AMFLS_LAUNCHED();
-        model_inner_kernel<<<ig, kThreads, 0, stream>>>(sums, chunks, outer, inner, w, w + 9,
+        model_inner_kernel<<<ig, kThreads, 0, stream>>>(sums, p.chunks, outer, inner, w, w + 9,
                                                         counter_, w + 5);
         AMFLS_LAUNCHED();
         // the reference's Frobenius bound sums column square sums: the inner
