@@ -41,7 +41,10 @@ inline int target_blocks() { return grid_cap(); }
 // shuffle tree per output was five FP64 additions per output and chunk on eight
 // multiply-adds (16384 x 512, four columns: 102 -> 65 us, one: 29 -> 24 us; eight outputs
 // for one column lost 3% on rows of 2000).  Its chunk minimum keeps those sums small
-// beside the products.
+// beside the products.  Where that gives fewer warps than the GPU has SM
+// quarters, a warp owns one output and half the chunk (three columns, 300 rows of
+// 40: 12.6 -> 4.6 us, 2000 of 120: 17.8 -> 6.7; two outputs with a tree each took
+// 7.5 and 10.6).
 constexpr int dot_outputs(int S) { return S >= 4 ? 2 : 4; }
 
 constexpr int pow2_ceil(int v) {
@@ -429,7 +432,10 @@ Split split_of(bool dot, int J, int min_rows, int out_n, int in_n) {
 // of a block product of S columns
 Split block_split(bool dot, int S, int out_n, int in_n) {
     if (!dot) return split_of(false, 1, 32, out_n, in_n);
-    return split_of(true, dot_outputs(S), 512, out_n, in_n);
+    const int J = dot_outputs(S);
+    const Split p = split_of(true, J, 512, out_n, in_n);
+    const long long warps = ((long long)out_n + J - 1) / J * p.chunks;
+    return warps >= 4LL * sm_count() ? p : split_of(true, 1, 256, out_n, in_n);
 }
 
 // of a double-double product
@@ -445,6 +451,9 @@ void launch_block(bool dot, const double* a, long long ld, int out_n, int in_n, 
     const dim3 grid(p.blocks_x, p.chunks);
     if (!dot)
         across_block_kernel<S><<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, p.chunk, x, ldx,
+                                                          partial, guard);
+    else if (p.J == 1)
+        dot_block_kernel<S, 1><<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, p.chunk, x, ldx,
                                                           partial, guard);
     else
         dot_block_kernel<S, dot_outputs(S)><<<grid, kThreads, 0, s>>>(a, ld, out_n, in_n, p.chunk,

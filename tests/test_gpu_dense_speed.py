@@ -1,6 +1,6 @@
-"""Dense products of many outputs with few chunks (across the contiguous
-dimension) keep the GPU busy: both directions read the same matrix, so that one
-does not take longer than the other.  Device times,
+"""Dense products of few outputs (along the contiguous dimension) and of many
+outputs with few chunks (across it) keep the GPU busy: both directions read the
+same matrix, so the one does not take longer than the other.  Device times,
 from products captured into a CUDA graph, the fastest of six replays."""
 import ctypes
 
@@ -46,6 +46,13 @@ def both(rows, cols, columns):
     a = torch.randn(rows, cols, dtype=torch.float64, device="cuda")
     along = product_us(amfls.DeviceOperator(a), rows, cols, columns)
     return along, product_us(amfls.DeviceOperator(a.t().contiguous().t()), rows, cols, columns)
+
+
+@pytest.mark.parametrize("rows,cols", [(40, 300), (120, 2000)])
+@pytest.mark.parametrize("columns", [2, 3])
+def test_few_outputs_along(rows, cols, columns):
+    along, across = both(rows, cols, columns)
+    assert along <= 1.15 * across
 
 
 @pytest.mark.parametrize("rows", [8192, 16384])
