@@ -255,7 +255,8 @@ public:
         : run_(run), lsmr_(lsmr) {
         ResidentOperator view;
         if (!op.resident(&view) || view.augmented ||
-            resident_excess(view) > kResidentIterationExcess)
+            resident_excess(view) > kResidentIterationExcess ||
+            !op.resident_tables(&view, run.stream()))
             return;
         grid_ = sm_count();
         args_.a = view.a;

@@ -60,6 +60,24 @@ double cost_estimate(const DeviceOperator& op) {
     return 4.0 * op.rows() * n;
 }
 
+// The resident kernels' tables of all problems, before the first solve: their
+// allocations would wait for the resident kernels of the others.
+void build_tables(const std::vector<BatchItem>& items) {
+    cudaStream_t s = nullptr;
+    for (const BatchItem& it : items) {
+        ResidentOperator view;
+        if (!resident_levels(*it.op, &view)) continue;
+        if (!s) AMFLS_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        try {
+            it.op->resident_tables(&view, s);
+        } catch (...) {
+            cudaStreamDestroy(s);
+            throw;
+        }
+    }
+    if (s) cudaStreamDestroy(s);
+}
+
 // SMs of each problem in LPT order (0: it has no resident levels), from the
 // batch alone (so that a repeat gives the same sums): of the `at_once` resident
 // problems that run from position p on, each takes the part of the SMs that the
@@ -141,13 +159,14 @@ std::vector<BatchOutcome> solve_amfls_batch(const std::vector<BatchItem>& items,
     });
     int device = 0;
     AMFLS_CUDA(cudaGetDevice(&device));
+    const auto t0 = std::chrono::steady_clock::now();
     const int at_once = std::min(workers, resident_streams());
+    build_tables(items);
     const std::vector<int> share = sm_shares(items, order, at_once);
     // workers beyond `at_once` take the other problems alone, on streams of
     // their own: the resident solves keep to as many streams as run at a time
     workers = std::min(workers, at_once + (int)std::count(share.begin(), share.end(), 0));
     Queue queue(share);
-    const auto t0 = std::chrono::steady_clock::now();
     auto work = [&](int w) {
         cudaStream_t s = nullptr;
         try {

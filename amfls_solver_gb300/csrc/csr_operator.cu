@@ -581,13 +581,15 @@ constexpr double kTuneMargin = 0.10;
 // runs).
 constexpr double kVectorMargin = 0.05;
 
-// Operators of at most this many nonzeros carry the sliced-row copy that the
-// resident kernels multiply by (two sides of 12 bytes a nonzero, up to a
-// quarter more for padding: 4 GB at the limit, and 9 bytes a row and column),
-// where the memory for it is there.  It pays at every size measured, up to the
-// 40 million nonzeros of the 2M x 500k matrix; beyond the limit the kernel chain
-// runs.  What else is allocated does not count: the tables decide the order of a
-// solve's sums.
+// Operators of at most this many nonzeros give the resident kernels a sliced-row
+// copy to multiply by (two sides of 12 bytes a nonzero, up to a quarter more for
+// padding: 4 GB at the limit, and 9 bytes a row and column), built by the first
+// solve that wants it where the memory is there: products alone need none, and
+// building it made the construction of an operator 15 to 25% longer (5000 x 1200
+// 640 -> 800 us, 60000 x 15000 5.8 -> 6.7 ms).  It pays at every size measured, up to
+// the 40 million nonzeros of the 2M x 500k matrix; beyond the limit the kernel
+// chain runs.  What else is allocated does not count: the tables decide the order
+// of a solve's sums.
 constexpr long long kResidentMaxNonzeros = 1LL << 27;
 
 struct CsrOperator::Side {
@@ -827,7 +829,7 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
     AMFLS_CUDA(cudaMemsetAsync(w, 0, sizeof(Work), stream));
     int *lens = nullptr, *bins = nullptr, *row_of = nullptr, *perm = nullptr, *counts = nullptr;
     const long long big = std::max<long long>(1, std::max<long long>(rows_, cols_));
-    AMFLS_CUDA(cudaMallocAsync(&lens, sizeof(int) * ((size_t)rows_ + cols_), stream));
+    AMFLS_CUDA(cudaMallocAsync(&lens, sizeof(int) * big, stream));
     AMFLS_CUDA(cudaMallocAsync(&bins, sizeof(int) * big, stream));
     AMFLS_CUDA(cudaMallocAsync(&row_of, sizeof(int) * std::max<long long>(1, nnz), stream));
     AMFLS_CUDA(cudaMallocAsync(&perm, sizeof(int) * std::max<long long>(1, nnz), stream));
@@ -905,7 +907,7 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
 
     // transpose bins
     check_offsets_kernel<<<setup_grid(cols_), 256, 0, stream>>>(
-        T.off, cols_, nnz, &w->err, &w->max_len_c, lens + rows_, elems_per_lane_, bins);
+        T.off, cols_, nnz, &w->err, &w->max_len_c, lens, elems_per_lane_, bins);
     AMFLS_LAUNCHED();
     build_bins(T, bins, stream);
     // int32 offsets and tilings of both sides for the streamed products
@@ -950,30 +952,40 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
     AMFLS_CUDA(cudaFreeAsync(row_of, stream));
     AMFLS_CUDA(cudaFreeAsync(perm, stream));
     AMFLS_CUDA(cudaFreeAsync(counts, stream));
-    // last, when all that the operator must have is there
-    try {
-        build_sliced_rows(lens, lens + rows_, stream);
-    } catch (...) {
-        stream_free(lens, stream);
-        throw;
-    }
     AMFLS_CUDA(cudaFreeAsync(lens, stream));
     AMFLS_CUDA(cudaStreamSynchronize(stream));
 }
 
+namespace {
+__global__ void row_lengths_kernel(const long long* off, int rows, int* lens) {
+    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < rows;
+         r += (long long)gridDim.x * blockDim.x)
+        lens[r] = (int)(off[r + 1] - off[r]);
+}
+}  // namespace
+
 // The tables of both sides, or none where the memory runs out.
-void CsrOperator::build_sliced_rows(const int* row_lens, const int* col_lens, cudaStream_t stream) {
-    if (nnz_ > kResidentMaxNonzeros) return;
-    const int per_lane = sliced::elements_per_lane(nnz_);
+void CsrOperator::build_sliced_rows(cudaStream_t stream) const {
+    int* lens = nullptr;
     try {
-        sliced::build(a_->rows, a_->off, a_->idx, a_->val, row_lens, rows_, per_lane, stream);
-        sliced::build(t_->rows, t_->off, t_->idx, t_->val, col_lens, cols_, per_lane, stream);
+        stream_alloc(&lens, sizeof(int) * (size_t)std::max(rows_, cols_), stream);
+        for (Side* s : {a_.get(), t_.get()}) {
+            row_lengths_kernel<<<setup_grid(s->count), 256, 0, stream>>>(s->off, s->count, lens);
+            AMFLS_LAUNCHED();
+            sliced::build(s->rows, s->off, s->idx, s->val, lens, s->count,
+                          sliced::elements_per_lane(nnz_), stream);
+        }
+        AMFLS_CUDA(cudaStreamSynchronize(stream));  // a solve on any stream may follow
     } catch (const CudaError& e) {
+        stream_free(lens, stream);
         a_->rows.release();
         t_->rows.release();
         if (e.code != cudaErrorMemoryAllocation) throw;
         cudaGetLastError();  // the failed allocation's
+        tables_missing_ = true;
+        return;
     }
+    stream_free(lens, stream);
 }
 
 namespace {
@@ -1117,14 +1129,21 @@ void CsrOperator::single_column_schedule(int chains[2], double microseconds[4]) 
 }
 
 bool CsrOperator::resident(ResidentOperator* view) const {
-    if (!a_->rows.tasks || !t_->rows.tasks) return false;
-    view->a = a_->rows.side;
-    view->t = t_->rows.side;
+    if (nnz_ > kResidentMaxNonzeros || tables_missing_) return false;
     view->rows = rows_;
     view->cols = cols_;
     view->nonzeros = nnz_;
     view->longest_row = max_row_nnz_;
     view->longest_col = max_col_nnz_;
+    return true;
+}
+
+bool CsrOperator::resident_tables(ResidentOperator* view, cudaStream_t stream) const {
+    if (!resident(view)) return false;
+    std::call_once(tables_built_, [&] { build_sliced_rows(stream); });
+    if (tables_missing_) return false;
+    view->a = a_->rows.side;
+    view->t = t_->rows.side;
     return true;
 }
 

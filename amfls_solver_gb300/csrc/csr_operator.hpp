@@ -1,9 +1,10 @@
 // FP64 CSR operator on the device (see csr_operator.cu).
 #pragma once
 
-#include <vector>
-
+#include <atomic>
 #include <memory>
+#include <mutex>
+#include <vector>
 
 #include "device_operator.hpp"
 
@@ -43,6 +44,7 @@ public:
     bool product1(bool transpose, const double* x, const Epilogue& ep,
                   cudaStream_t s) const override;
     bool resident(ResidentOperator* view) const override;
+    bool resident_tables(ResidentOperator* view, cudaStream_t s) const override;
     // Tiling of the single-column products per side (A, then the stored
     // transpose): 1 = chain groups, 0 = row blocks; the autotuner's timings
     // (microseconds per product, row blocks then chain groups, 0 = not timed).
@@ -53,7 +55,7 @@ private:
     struct Side;
     void build(const long long* d_off, const long long* d_idx, const double* d_val,
                cudaStream_t stream);
-    void build_sliced_rows(const int* row_lens, const int* col_lens, cudaStream_t stream);
+    void build_sliced_rows(cudaStream_t stream) const;
     void build_bins(Side& s, const int* d_bins, cudaStream_t stream);
     void tune_single_column(Side& s, const std::vector<long long>& host_off,
                             cudaStream_t stream);
@@ -78,6 +80,10 @@ private:
     // row-major staging of a multi-column input block (max(rows, cols) x 8);
     // multi-column products on one operator are therefore stream-ordered
     double* xrows_ = nullptr;
+    // the resident kernels' tables (Side::rows): built once, or found to have no
+    // memory, whichever solve comes first
+    mutable std::once_flag tables_built_;
+    mutable std::atomic<bool> tables_missing_{false};
 };
 
 // The matrix of a CsrOperator with its values rounded to FP32 or BF16 (one

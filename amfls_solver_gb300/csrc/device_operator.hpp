@@ -123,10 +123,16 @@ public:
         (void)transpose; (void)x; (void)ep; (void)s;
         return false;
     }
-    // The tables with which the resident level kernel computes the products
-    // itself; false when the operator has none.
+    // Whether the resident kernels can compute the products themselves, from
+    // tables that the operator has or would build; `view` gets the sizes.
     virtual bool resident(ResidentOperator* view) const {
         (void)view;
+        return false;
+    }
+    // The same with the tables, which the first call builds on `s` and waits
+    // for; false where there is no memory for them.
+    virtual bool resident_tables(ResidentOperator* view, cudaStream_t s) const {
+        (void)view; (void)s;
         return false;
     }
     // Storage kind for diagnostics: 0 CSR, 1 row-major dense, 2 column-major

@@ -442,11 +442,24 @@ void AugmentedOperator::apply_transpose(const double* y, int block_cols, double*
     }
 }
 
-bool AugmentedOperator::resident(ResidentOperator* view) const {
-    if (!a_.resident(view) || view->augmented) return false;
-    view->augmented = true;
-    view->root = root_;
+bool AugmentedOperator::augment(bool there, ResidentOperator& inner, ResidentOperator* view) const {
+    if (!there || inner.augmented) return false;
+    inner.augmented = true;
+    inner.root = root_;
+    *view = inner;
     return true;
+}
+
+bool AugmentedOperator::resident(ResidentOperator* view) const {
+    ResidentOperator inner;
+    const bool there = a_.resident(&inner);
+    return augment(there, inner, view);
+}
+
+bool AugmentedOperator::resident_tables(ResidentOperator* view, cudaStream_t s) const {
+    ResidentOperator inner;
+    const bool there = a_.resident_tables(&inner, s);
+    return augment(there, inner, view);
 }
 
 bool AugmentedOperator::product1(bool transpose, const double* x, const Epilogue& ep,

@@ -76,8 +76,10 @@ public:
     bool product1(bool transpose, const double* x, const Epilogue& ep,
                   cudaStream_t s) const override;
     bool resident(ResidentOperator* view) const override;
+    bool resident_tables(ResidentOperator* view, cudaStream_t s) const override;
 
 private:
+    bool augment(bool there, ResidentOperator& inner, ResidentOperator* view) const;
     const DeviceOperator& a_;
     double root_;
     ValidationModel model_;

@@ -1668,7 +1668,7 @@ void Workspace::advance_to(int target_depth) {
     if (V32_) V32_->ensure_columns(host_.k + levels + 1);
     if (V16_) V16_->ensure_columns(host_.k + levels + 1);
     interval_graph_ = false;
-    if (resident_grid_ > 0 && host_.k + levels <= kResidentMaxBasis) {
+    if (resident_grid_ > 0 && host_.k + levels <= kResidentMaxBasis && resident_ready()) {
         run_resident(levels, target_depth);
         return;
     }
@@ -1700,6 +1700,13 @@ int Workspace::resident_interval_grid() const {
     int grid = resident_grid_;
     for (long long k = kGrowBasis; k <= host_.k && grid < sm_count(); k *= 2) grid *= 2;
     return std::min(grid, sm_count());
+}
+
+// The operator's tables are there: the first solve with an interval of
+// width-one levels builds them.
+bool Workspace::resident_ready() {
+    if (!resident_op_.a.tasks && !op_.resident_tables(&resident_op_, stream_)) resident_grid_ = 0;
+    return resident_grid_ > 0;
 }
 
 void Workspace::run_resident(int levels, int target_depth) {

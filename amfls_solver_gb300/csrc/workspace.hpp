@@ -134,6 +134,7 @@ private:
     void release() noexcept;
     void enqueue_level_kernels(cudaStream_t s, int pcap);
     int resident_interval_grid() const;
+    bool resident_ready();
     void run_resident(int levels, int target_depth);
     void build_graph(int pcap);
     void invalidate_graph();

@@ -1,7 +1,8 @@
 """The sliced-row tables are an extra of a CSR operator, without a GPU: the
 operator's object file linked against a stand-in for the CUDA runtime (memory on
 the host, kernels that do nothing) and for the tables' construction, which runs
-out of memory on either side or fails otherwise."""
+out of memory on either side or fails otherwise.  They are built when a solve
+first asks for them, once."""
 import subprocess
 
 import pytest
@@ -120,7 +121,11 @@ int main() {
         try {
             CsrOperator op(3, 2, off, idx, val, 6, nullptr);
             ResidentOperator view;
-            std::printf("%d %d %d\n", op.resident(&view) ? 1 : 0, released, (int)last);
+            const int sizes = op.resident(&view), early = calls;
+            const int first = op.resident_tables(&view, nullptr);
+            const int again = op.resident_tables(&view, nullptr);
+            std::printf("%d %d %d%d %d %d %d\n", sizes, early, first, again, calls, released,
+                        (int)last);
         } catch (const std::exception&) {
             std::printf("raised %d\n", released);
         }
@@ -145,13 +150,19 @@ def outcomes(tmp_path_factory):
     return run.stdout.splitlines()
 
 
+def test_tables_are_built_once_and_when_asked_for(outcomes):
+    """Sizes known, no table before the first request, two sides after it."""
+    assert outcomes[0] == "1 0 11 2 0 0"
+
+
 def test_tables_do_not_depend_on_the_free_memory(outcomes):
-    assert outcomes[:2] == ["1 0 0", "1 0 0"]
+    assert outcomes[1] == outcomes[0]
 
 
-def test_an_operator_without_memory_for_tables_is_built_without_them(outcomes):
-    """No side's table is left, and no error for the next call to find."""
-    assert outcomes[2:4] == ["0 0 0", "0 1 0"]
+def test_an_operator_without_memory_for_tables_does_without_them(outcomes):
+    """No side's table is left, no further attempt, and no error for the next
+    call to find."""
+    assert outcomes[2:4] == ["1 0 00 1 0 0", "1 0 00 2 1 0"]
 
 
 def test_other_failures_are_raised(outcomes):
