@@ -363,11 +363,8 @@ tile_product_kernel(const int* __restrict__ off, const int* __restrict__ idx,
 #pragma unroll
                 for (int u = 0; u < kStep; ++u)
                     xv[u] = jv[u] >= 0 ? to_acc<A>(__ldg(x + (long long)jv[u] * C + cl)) : A(0);
-                // a step beyond the row's end would take its slot of the FP64
-                // pipe all the same (rows of 80: 20 steps, not 32)
 #pragma unroll
-                for (int u = 0; u < kStep; ++u)
-                    if (base + kG * u < d.w) part = fma(av[u], xv[u], part);
+                for (int u = 0; u < kStep; ++u) part = fma(av[u], xv[u], part);
             }
             for (int o = 16; o >= C; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
             double acc[C];
