@@ -19,16 +19,17 @@ e2e       the same solve through the public API run_amfls on pinned host
           tensors: host->device copies of the CSR arrays and b, operator
           construction (transpose, task tables, certified norm model), solve,
           device->host copy of the solution;
-roofline  the dominant kernels of the solve, the width-one
-          reorthogonalisation sweeps (c = V^T r and r -= V c over the basis V),
-          timed live with CUDA events on their stream at the solve's mean basis
-          size; algorithmic bytes 8 n k + 8 n (+ 8 n for the update);
+roofline  the timed solve itself, nearly all of it one kernel
+          (resident_levels_kernel, a checkpoint interval of levels a launch):
+          the algorithmic bytes of its levels (the basis V twice a level,
+          c = V^T r and r -= V c, and the two products) over the solve's time,
+          and its FP64 multiply-adds over what the FP64 pipe can do;
 c3        time-to-tol on the 2,000,000 x 500,000 power-law CSR problem
           (lambda = 1e-4, tol = 1e-10; the metric's target workload): plain
           FP64 and the chosen form (FP64 residual correction around restart
           cycles with reduced-basis sweeps), status, depth, certificate, time
           split, speed-up, x against plain FP64's, and the roofline of each
-          form's dominant sweeps;
+          form's solve;
 dense     the 100000 x 2000 column-major dense operator (lambda = 1e-6,
           tol = 1e-10): plain FP64 and the mixed form;
 spmm      CSR SpMM / SpMM^T GB/s (s = 1 and 8) on the 2M x 500k matrix;
@@ -70,9 +71,8 @@ SEED = 20251203
 C3_CYCLE = 2000  # restart-cycle length of the chosen form on the 2M x 500k problem
 C3_STORAGE = "fp16"  # precision of the chosen form's copy of the basis ("fp32" or "fp16")
 C3_STORAGE_CODE = {"fp32": 1, "fp16": 2}[C3_STORAGE]
-# DRAM bytes of one V^T r + r - V c pair measured by ncu (--set full) on the
-# warp-task sweeps at n = 5000, k = 1900: 76.875 + 1.307 MB and 76.860 + 1.436 MB
-SWEEP_CAPTURE = {"n": 5000, "k": 1900, "bytes": (76.875 + 1.307 + 76.860 + 1.436) * 1e6}
+# FP64 multiply-adds per second of the chip: two lanes per SM clock
+FP64_FMA_RATE = 152 * 2 * 2.07e9
 
 
 def parse():
@@ -229,48 +229,26 @@ def cpu_baseline(prob, opts, name):
 
 # ------------------------------------------------------------ GPU legs ----
 
-def reorth_roofline(lib, n, k, stream, peak, peak_kind):
-    """The width-one reorthogonalisation sweeps timed live on `stream` at
-    basis size k (amfls_gpu_probe_reorthogonalization: the solver's own
-    kernels on its panel layout, CUDA events around each kind)."""
-    import ctypes
-    from amfls_solver_gb300 import _native
-    secs = (ctypes.c_double * 2)()
-    _native.check(lib.amfls_gpu_probe_reorthogonalization(n, k, 50, ctypes.c_void_p(stream),
-                                                          secs))
-    vt, vc = secs[0], secs[1]
-    bytes_vt = 8.0 * n * k + 8.0 * n * ((k + 31) // 32)  # V once, r once per panel
-    bytes_vc = 8.0 * n * k + 16.0 * n                    # V once, r in and out
-    achieved = (bytes_vt + bytes_vc) / (vt + vc) / 1e9
-    return {"kernel": "vt_r_kernel (c = V^T r) + v_c_kernel (r -= V c)", "bound": "hbm",
-            "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "peak_source": peak_kind, "traffic": None, "basis_rows": n, "basis_cols": k,
-            "launch_us": {"vt_r": vt * 1e6, "v_c": vc * 1e6},
-            "algorithmic_bytes": {"vt_r": bytes_vt, "v_c": bytes_vc}}
-
-
-def reduced_reorth_roofline(lib, n, k, stream, peak, peak_kind, storage):
-    """The reduced-basis sweeps (an FP32 (storage 1) or FP16 (2) copy of V:
-    c = V~^T r~, r -= fl64(V~ c~)) timed live on `stream` at basis size k
-    (amfls_gpu_probe_reorthogonalization_reduced)."""
-    import ctypes
-    from amfls_solver_gb300 import _native
-    secs = (ctypes.c_double * 2)()
-    err = ctypes.c_double()
-    _native.check(lib.amfls_gpu_probe_reorthogonalization_reduced(
-        n, k, 50, storage, ctypes.c_void_p(stream), secs, ctypes.byref(err)))
-    vt, vc = secs[0], secs[1]
-    e = 4.0 if storage == 1 else 2.0                    # bytes per element of V~
-    bytes_vt = e * n * k + 4.0 * n * ((k + 31) // 32)  # V~ once, r~ once per panel
-    bytes_vc = e * n * k + 16.0 * n                    # V~ once, r in and out
-    achieved = (bytes_vt + bytes_vc) / (vt + vc) / 1e9
-    return {"kernel": ("vt_r32_kernel (c = V~^T r~) + v_c32_kernel (r -= fl64(V~ c~)), "
-                       f"{'FP32' if storage == 1 else 'FP16'} copy of V"),
-            "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak, "peak_source": peak_kind, "traffic": None,
-            "basis_rows": n, "basis_cols": k, "launch_us": {"vt_r32": vt * 1e6, "v_c32": vc * 1e6},
-            "algorithmic_bytes": {"vt_r32": bytes_vt, "v_c32": bytes_vc},
-            "max_coefficient_error_rel_r": err.value}
+def solve_roofline(seconds, rows, cols, nnz, levels, peak, peak_kind, cycles=1, element=8):
+    """A solve of `levels` width-one levels in `cycles` runs from an empty
+    basis: per level the basis is read twice (c = V^T r, r -= V c; `element`
+    bytes an entry) and A and A^T once (12 bytes a nonzero), against the whole
+    solve's time, checkpoints included.  Second projection passes, where the
+    DGKS test asks for them, are not counted."""
+    per = levels / cycles
+    sweeps = cycles * element * cols * per * per
+    products = levels * (24.0 * nnz + 16.0 * (rows + cols))
+    achieved = (sweeps + products) / seconds / 1e9
+    out = {"kernel": "resident_levels_kernel (both products and both sweeps of every level)",
+           "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+           "frac": achieved / peak, "peak_source": peak_kind, "traffic": None,
+           "seconds": seconds, "levels": levels, "cycles": cycles,
+           "algorithmic_bytes": {"sweeps": sweeps, "products": products}}
+    if element == 8:
+        fma = sweeps / 8 + 2.0 * nnz * levels
+        out["fp64_fma"] = {"count": fma, "rate": fma / seconds,
+                           "frac": fma / seconds / FP64_FMA_RATE}
+    return out
 
 
 def spmm_measurement(dev, stream, peak):
@@ -663,20 +641,10 @@ def run_ours(args, world, rank, local):
     e2e = statistics.mean(e2e_times)
 
     peak, peak_kind = measured_peaks()
-    roof = reorth_roofline(lib, prob.cols, max(32, depth // 2), stream.cuda_stream, peak,
-                           peak_kind)
-    roof["note"] = ("kernels at the solve's mean basis size (depth / 2 columns); the "
-                    "operator products of this problem are latency-bound single-column "
-                    "SpMVs (spmm carries the HBM-bound ones)")
-    if prob.cols == SWEEP_CAPTURE["n"]:
-        # DRAM bytes of the pair from one ncu capture of the same kernels at
-        # n = 5000, k = 1900 (the only traffic figure a live run cannot read),
-        # scaled to this basis size
-        k = roof["basis_cols"]
-        roof["traffic"] = SWEEP_CAPTURE["bytes"] * k / SWEEP_CAPTURE["k"]
-        roof["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of "
-                                  "sweep_vt_kernel + sweep_vc_kernel at n = 5000, k = 1900, "
-                                  "scaled by k")
+    roof = solve_roofline(t_step, prob.rows, prob.cols, prob.nnz, depth, peak, peak_kind)
+    roof["note"] = ("the basis of this problem (up to 151 MB) stays largely in L2: an interval of "
+                    "512 levels at 1536 to 2048 columns read 4.3 GB from DRAM for 73 GB of sweeps "
+                    "(ncu); FP64 operations and the grid-wide steps between phases bound it")
 
     legs = {}
     if rank == 0:
@@ -693,13 +661,13 @@ def run_ours(args, world, rank, local):
         if args.c3:
             c3, _ = c3_measurement(dev)
             if "fp64" in c3 and "depth" in c3["fp64"]:
-                c3["roofline"] = reorth_roofline(lib, c3["cols"], max(32, c3["fp64"]["depth"] // 2),
-                                                 stream.cuda_stream, peak, peak_kind)
+                c3["roofline"] = solve_roofline(c3["fp64"]["s"], c3["rows"], c3["cols"], c3["nnz"],
+                                                c3["fp64"]["depth"], peak, peak_kind)
+                c3["roofline"]["note"] = "beyond 10240 columns the kernel chain runs the levels"
             if "mixed" in c3:
-                c3["mixed"]["roofline"] = reduced_reorth_roofline(
-                    lib, c3["cols"], C3_CYCLE // 2, stream.cuda_stream, peak, peak_kind,
-                    C3_STORAGE_CODE)
-                c3["mixed"]["roofline"]["note"] = "at the mean basis size of a restart cycle"
+                c3["mixed"]["roofline"] = solve_roofline(
+                    c3["mixed"]["s"], c3["rows"], c3["cols"], c3["nnz"], c3["mixed"]["depth"], peak,
+                    peak_kind, c3["mixed"]["cycles"], {1: 4, 2: 2}[C3_STORAGE_CODE])
             legs["c3"] = c3
     if rank != 0:
         return
