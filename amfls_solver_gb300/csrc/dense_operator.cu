@@ -172,44 +172,57 @@ __global__ void reduce_block_kernel(const double* partial, int chunks, int S, in
     }
 }
 
+// kSliced false: the chunk sums of an AMFLS level's product (see product1).
+template <bool kSliced>
 __global__ void __launch_bounds__(kThreads)
 reduce_sliced_kernel(const double* __restrict__ partial, int chunks, int S, int outer, double* y,
-                     long long ldy, const int* guard) {
+                    long long ldy, const int* guard) {
     __shared__ double slice[kThreads / 32][kSliceOutputs];
     if (guard && *guard == 0) return;
     const long long total = (long long)S * outer;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int kSlices = kThreads / kSliceOutputs;
-    for (long long t0 = (long long)blockIdx.x * kSliceOutputs; t0 < total;
-         t0 += (long long)gridDim.x * kSliceOutputs) {
-        const long long t = t0 + lane % kSliceOutputs;
-        double x[4] = {0.0, 0.0, 0.0, 0.0};
-        if (t < total) {
-            const double* p = partial + t;
-            int ch = threadIdx.x / kSliceOutputs;
-            for (; ch + 3 * kSlices < chunks; ch += 4 * kSlices) {
-                double v[4];
+    auto put = [&](long long t, double v) {
+        const int c = (int)(t / outer);
+        y[t - (long long)c * outer + c * ldy] = v;
+    };
+    if constexpr (kSliced) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        constexpr int kSlices = kThreads / kSliceOutputs;
+        for (long long t0 = (long long)blockIdx.x * kSliceOutputs; t0 < total;
+             t0 += (long long)gridDim.x * kSliceOutputs) {
+            const long long t = t0 + lane % kSliceOutputs;
+            double x[4] = {0.0, 0.0, 0.0, 0.0};
+            if (t < total) {
+                const double* p = partial + t;
+                int ch = threadIdx.x / kSliceOutputs;
+                for (; ch + 3 * kSlices < chunks; ch += 4 * kSlices) {
+                    double v[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) v[u] = p[(ch + u * kSlices) * total];
+                    for (int u = 0; u < 4; ++u) v[u] = p[(ch + u * kSlices) * total];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) x[u] += v[u];
+                    for (int u = 0; u < 4; ++u) x[u] += v[u];
+                }
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if (ch + u * kSlices < chunks) x[u] += p[(ch + u * kSlices) * total];
             }
-#pragma unroll
-            for (int u = 0; u < 3; ++u)
-                if (ch + u * kSlices < chunks) x[u] += p[(ch + u * kSlices) * total];
+            double v = (x[0] + x[1]) + (x[2] + x[3]);
+            v += __shfl_xor_sync(0xffffffffu, v, 8);
+            v += __shfl_xor_sync(0xffffffffu, v, 16);
+            if (lane < kSliceOutputs) slice[warp][lane] = v;
+            __syncthreads();
+            if (threadIdx.x < kSliceOutputs && t < total)
+                put(t, ((slice[0][lane] + slice[1][lane]) + (slice[2][lane] + slice[3][lane])) +
+                           ((slice[4][lane] + slice[5][lane]) +
+                            (slice[6][lane] + slice[7][lane])));
+            __syncthreads();
         }
-        double v = (x[0] + x[1]) + (x[2] + x[3]);
-        v += __shfl_xor_sync(0xffffffffu, v, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        if (lane < kSliceOutputs) slice[warp][lane] = v;
-        __syncthreads();
-        if (threadIdx.x < kSliceOutputs && t < total) {
-            const int c = (int)(t / outer);
-            y[t - (long long)c * outer + c * ldy] =
-                ((slice[0][lane] + slice[1][lane]) + (slice[2][lane] + slice[3][lane])) +
-                ((slice[4][lane] + slice[5][lane]) + (slice[6][lane] + slice[7][lane]));
+    } else {
+        for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+             t += (long long)gridDim.x * blockDim.x) {
+            double s = partial[t];
+            for (int ch = 1; ch < chunks; ++ch) s += partial[ch * total + t];
+            put(t, s);
         }
-        __syncthreads();
     }
 }
 
@@ -446,7 +459,7 @@ Split refined_split(bool dot, int out_n, int in_n) {
 template <int S>
 void launch_block(bool dot, const double* a, long long ld, int out_n, int in_n, const double* x,
                   long long ldx, double* partial, double* y, long long ldy, cudaStream_t s,
-                  const int* guard = nullptr, bool slices = true) {
+                  const int* guard = nullptr, bool level = false) {
     const Split p = block_split(dot, S, out_n, in_n);
     const dim3 grid(p.blocks_x, p.chunks);
     if (!dot)
@@ -460,10 +473,13 @@ void launch_block(bool dot, const double* a, long long ld, int out_n, int in_n, 
                                                                        x, ldx, partial, guard);
     AMFLS_LAUNCHED();
     const long long total = (long long)S * out_n;
-    if (slices && sliced_sums(total, p.chunks)) {
+    if (S == 1 && level) {
+        reduce_sliced_kernel<false><<<grid_1d(total), kThreads, 0, s>>>(partial, p.chunks, S, out_n,
+                                                                        y, ldy, guard);
+    } else if (sliced_sums(total, p.chunks)) {
         const long long groups = (total + kSliceOutputs - 1) / kSliceOutputs;
-        reduce_sliced_kernel<<<(int)std::min<long long>(groups, target_blocks()), kThreads, 0, s>>>(
-            partial, p.chunks, S, out_n, y, ldy, guard);
+        reduce_sliced_kernel<true><<<(int)std::min<long long>(groups, target_blocks()), kThreads, 0,
+                                     s>>>(partial, p.chunks, S, out_n, y, ldy, guard);
     } else {
         reduce_block_kernel<<<grid_1d(total), kThreads, 0, s>>>(partial, p.chunks, S, out_n, y, ldy,
                                                                 guard);
@@ -616,16 +632,18 @@ bool DenseOperator::product1(bool transpose, const double* x, const Epilogue& ep
     // contiguous (apply = dot of rows); column-major columns are (transpose =
     // dot of columns).
     //
-    // A level's product goes without the sliced sums: the width controller weighs
-    // its measured cost against the local algebra, and the policies trained on
-    // the controller's decisions earn their gain where it widens.  With the sliced
-    // sums (131 -> 27 us, 16384 x 512 transposed) it never widens on the dense
-    // study family, and a policy has nothing left to gain there.
+    // A level's product keeps slower chunk sums (16384 x 512 transposed: 134 us, 72
+    // with reduce_block_kernel's, 27 sliced): the width controller weighs its
+    // measured cost against the local algebra, and the policies trained on the
+    // controller's decisions depend on it.  On the dense study family the
+    // trained policy gains 34 to 44% against the heuristic with these sums;
+    // with those of 72 us anything from 41 to -50%, as where the gate stops
+    // widening there is little left to learn.
     const int out_n = transpose ? cols_ : rows_;
     const int in_n = transpose ? rows_ : cols_;
     const long long ld = column_major_ ? rows_ : cols_;
     launch_block<1>(column_major_ == transpose, a_, ld, out_n, in_n, x, in_n, partials_, tmp_,
-                    out_n, s, ep.guard, !ep.level);
+                    out_n, s, ep.guard, ep.level);
     run_epilogue(tmp_, out_n, ep, ep.partials ? ep.partials : scratch_,
                  ep.counter ? ep.counter : counter_ + 1, s);
     return true;
