@@ -11,7 +11,8 @@
 // that leaves most of a whole GPU idle, and its work takes no longer on ten
 // SMs than it waits anyway.  Sixteen CSR problems of up to 20000 x 4000, 16
 // workers: 337 ms with the level kernels launched from the host, 261 ms with
-// the waits of the validation taken out, 128 ms with the shares.  Other operators'
+// the waits of the validation taken out, 128 ms with the shares, 114 ms with
+// shares that grow with the basis (Workspace::resident_interval_grid).  Other operators'
 // levels are launched from the host when there is more than one worker
 // (graphs of different streams ran one at a time: 48 problems, 16 workers,
 // 12.5 s against 7.9 s).

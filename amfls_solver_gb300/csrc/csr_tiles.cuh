@@ -92,9 +92,9 @@ constexpr int kRowBlock = -64, kWholeRow = -2, kChainGroup = -3;
 // takes as many FP64 steps as its longest row, and an idle lane's step takes
 // the pipe's time all the same; the bit is set where the split saves a fifth of
 // the block's steps.  Microseconds per product without and with it: 33 nonzeros in
-// every row, so that a block holds one (50000 x 12000), 105 and 60 for 8
-// columns, 100 and 39 for 2; power-law rows (200000 x 50000, 20 on average) 93 and 91
-// for 8, 66 and 60 for 4.
+// every row, so that a block holds one (50000 x 12000), 97.7 and 51.7 for 8
+// columns, 92 and 28 for 2; power-law rows (200000 x 50000, 20 on average) 87.5 and
+// 82.7 for 8, 55.9 and 50.6 for 4.
 constexpr int split_bit(int c) { return c == 2 ? 1 : c == 4 ? 2 : 4; }
 constexpr bool is_row_block(int q) { return q <= kRowBlock + 7; }
 

@@ -7,11 +7,11 @@
 // cooperative kernel with one block of 384 threads on each SM of its grid (512
 // threads spill registers and 256 leave too few gathers in flight: 129 us per
 // level of a 200000 x 50000 power-law problem against 139 and 148).
-// Whole solves, kernel chain -> resident: 2000 x 500 28.7 -> 14.8 ms,
-// 20000 x 5000 142 -> 80.6 ms, 60000 x 15000 274 -> 172 ms, the mixed form on
-// 200000 x 50000 565 -> 267 ms.  It stays ahead up to the 2M x 500k matrix
-// (500 levels: 1253 -> 1207 us per level FP64, 967 -> 780 us on the FP16 copy),
-// so every CSR operator that carries the tables uses it.
+// Whole solves, kernel chain -> now: 2000 x 500 28.7 -> 10.0 ms, 20000 x 5000 142 ->
+// 65 ms, 60000 x 15000 274 -> 160 ms, the mixed form on 200000 x 50000 565 -> 242 ms.  It
+// stays ahead up to the 2M x 500k matrix (500 levels: 1253 -> 1207 us per level FP64,
+// 967 -> 780 us on the FP16 copy), so operators that have the tables use it but for
+// those with rows far longer than the others (resident_excess).
 // A level (krylov_workspace.cpp:589-831) is five phases with a grid barrier
 // after each:
 //   1  u = y / ||y|| (the previous level's), r = A^T u - beta v
@@ -81,7 +81,7 @@ static_assert(offsetof(Shared, seg) % 16 == 0 && kW <= 16);
 // Each warp owns kSlots slots of 4 KB and is its own producer: bulk copies
 // bring the next pieces of the basis while the current one is multiplied, and
 // the first pieces of a sweep before the grid barrier in front of it (V does
-// not change while r or c is formed).  The 128 KB on their way per SM cover the
+// not change while r or c is formed).  The 96 KB on their way per SM cover the
 // memory's latency at the FP64 pipe's rate without holding registers.
 
 struct Ring {
