@@ -862,6 +862,7 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
     AMFLS_CUDA(cudaStreamSynchronize(stream));
     if (err & 4) fail("CSR column index is out of range");
     if (err & 8) fail("CSR values must be finite");
+
     // transpose: stable sort of entry ids by column
     AMFLS_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (cols_ + 1), stream));
     if (nnz > 0) {
@@ -910,6 +911,7 @@ void CsrOperator::build(const long long* d_off, const long long* d_idx, const do
         T.off, cols_, nnz, &w->err, &w->max_len_c, lens, elems_per_lane_, bins);
     AMFLS_LAUNCHED();
     build_bins(T, bins, stream);
+
     // int32 offsets and tilings of both sides for the streamed products
     for (Side* sd : {&A, &T}) {
         narrow_offsets_kernel<<<setup_grid(sd->count + 1), 256, 0, stream>>>(sd->off, sd->count,

@@ -168,7 +168,7 @@ struct Store {
 };
 
 // Builds the table of a side from its CSR arrays (device), on `stream`;
-// synchronises once to size the copy.  `lens` holds the row lengths.
+// synchronises twice to size the copy.  `lens` holds the row lengths.
 void build(Store& store, const long long* off, const int* idx, const double* val,
            const int* lens, int count, int per_lane, cudaStream_t stream);
 
